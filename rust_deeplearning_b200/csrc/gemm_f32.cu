@@ -1,61 +1,378 @@
 // Matrix product of the 32-bit path: out[m, n] = sum_k x[m, k] * w[n, k], float operands, fused
-// multiply-add in float, no tensor cores and no reduced-precision mode.  Every output element is
-// summed over k = 0 .. K-1 in that order, whatever M, N or the element's place in a tile, so a
-// row's result does not depend on which other rows are in the batch.
+// multiply-add in float, no tensor cores and no reduced-precision mode.
+//
+// Every output element is summed in one order that depends on K alone, whatever M, N or the element's
+// place in a tile, so a row's result does not depend on which other rows are in the batch: k is cut into
+// eight runs of equal length (a multiple of four); inside a run two chains of fused multiply-adds take the
+// even and the odd k (the halves of the two-wide instruction) and are added at the run's end; the runs' sums
+// are added one after another.  (One chain over all k, as before, is 2.0 to 2.6 times further from the 64-bit
+// result.)  Zeros stand in for k beyond a run: they change no chain.
+//
+// Two kernels share that order.
+//   * Up to 16 rows the weights' bytes bound the product (10.4 GB a step at the 2B shape).  A warp takes one run of k
+//     of a tile of 32 or 16 weight rows - a lane a row, its sums over all x rows in registers - through a ring of its
+//     own in shared memory (cp.async, 16 bytes a lane, rows 144 bytes apart so that a quarter warp's reads fall into
+//     different banks); the eight warps of a block are the eight runs, whose sums meet in shared memory once a tile.
+//     Blocks are persistent and the ring runs on from tile to tile; weights are asked for before the wait on the
+//     kernel before.
+//   * Above, the float units bound it.  A block forms a tile of 32, 48, 64 or 128 rows by 128 columns, a thread 2 to 8 by 8
+//     of them, both operands' rows in shared memory as they lie in memory (no transposition: the two-wide instruction
+//     takes neighbouring k).  Where the tiles alone do not fill the chip, eight blocks (a cluster) share a tile, a run of k
+//     each, and add up through distributed shared memory.
+// Both take operands that are not 16-byte aligned (or K not a multiple of four) by 4-byte copies.
 // (The reference's product is an f32 library GEMM: rustml/core/main/src/core/tensor/ops.rs:806-823;
 // y = x W^T with W [out, in]: rustml/nn/main/src/core/linear.rs:12-15, :168-169.)
 #include "api.h"
 #include "common.cuh"
+#include "launch.cuh"
 
 namespace {
 
-constexpr int TM = 64, TN = 64, TK = 16;
+constexpr int RUNS = 8;             // runs of k
+constexpr int KC = 32;              // k of a chunk in shared memory
+constexpr int PITCH = KC + 4;       // floats between the rows of a chunk
 
-__global__ void __launch_bounds__(256) gemm_f32_kernel(float* __restrict__ out, const float* __restrict__ x,
-                                                       const float* __restrict__ w, int M, int N, int K) {
-    __shared__ float xs[TK][TM + 1];
-    __shared__ float ws[TK][TN + 1];
-    const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // 16 x 16 threads, 4 x 4 outputs each
-    float acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+// Length of a run of k: a multiple of four, eight of them cover K.
+__host__ __device__ __forceinline__ int run_length(int K) { return ((K + RUNS - 1) / RUNS + 3) & ~3; }
 
-    for (int k0 = 0; k0 < K; k0 += TK) {
-        // 64 rows x 16 k of each operand: 1024 values, 4 per thread, k fastest for coalescing
-        for (int idx = threadIdx.x; idx < TM * TK; idx += 256) {
-            const int r = idx / TK, kk = idx - r * TK;
-            const int gm = m0 + r, gn = n0 + r, gk = k0 + kk;
-            xs[kk][r] = (gm < M && gk < K) ? x[(long long)gm * K + gk] : 0.f;
-            ws[kk][r] = (gn < N && gk < K) ? w[(long long)gn * K + gk] : 0.f;
-        }
-        __syncthreads();
+__device__ __forceinline__ unsigned long long ffma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ float halves_sum(unsigned long long v) {
+    return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32));
+}
+struct Pairs { unsigned long long lo, hi; };        // four neighbouring k
+__device__ __forceinline__ Pairs lds_pairs(uint32_t addr) {
+    Pairs v;
+    asm volatile("ld.shared.v2.u64 {%0,%1}, [%2];" : "=l"(v.lo), "=l"(v.hi) : "r"(addr));
+    return v;
+}
+// Four floats from p (n of them exist, the rest become zero) to shared memory.
+template <bool ALIGNED>
+__device__ __forceinline__ void copy4(uint32_t dst, const float* p, int n) {
+    if (ALIGNED) {
+        const int bytes = n > 0 ? 16 : 0;            // K and the runs are multiples of four
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(p), "r"(bytes) : "memory");
+    } else {
 #pragma unroll
-        for (int kk = 0; kk < TK; ++kk) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = xs[kk][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = ws[kk][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int gm = m0 + ty * 4 + i;
-        if (gm >= M) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int gn = n0 + tx * 4 + j;
-            if (gn < N) out[(long long)gm * N + gn] = acc[i][j];
+        for (int i = 0; i < 4; ++i) {
+            const int bytes = i < n ? 4 : 0;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + 4 * i), "l"(i < n ? p + i : p), "r"(bytes) : "memory");
         }
     }
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
+
+// ---- few rows ----
+
+// ROWS weight rows a tile (16: half a warp each takes half of the x rows), MT x rows, STAGES chunks of a warp's ring.
+template <int ROWS, int MT, int STAGES, bool ALIGNED>
+__global__ void __launch_bounds__(RUNS * 32, 1) gemm_f32_few_kernel(float* __restrict__ out, const float* __restrict__ x,
+                                                                   const float* __restrict__ w, int M, int N, int K) {
+    constexpr int MINE = ROWS == 32 ? MT : MT / 2;           // x rows of a lane
+    constexpr int STAGE = ROWS * PITCH + MT * KC;            // floats
+    extern __shared__ __align__(16) float ring[];
+    __shared__ float part[2][RUNS][MT][ROWS];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int row = ROWS == 32 ? lane : lane & 15, m0 = ROWS == 32 ? 0 : (lane >> 4) * MINE;
+    const int run = run_length(K), k_lo = warp * run, k_hi = min(K, k_lo + run);
+    const int chunks = k_hi > k_lo ? (k_hi - k_lo + KC - 1) / KC : 0;
+    const int n_tiles = (N + ROWS - 1) / ROWS;
+    const uint32_t mine = (uint32_t)__cvta_generic_to_shared(ring) + (uint32_t)(warp * STAGES * STAGE * 4);
+
+    auto copy_w = [&](int tile, int c, int s) {
+        const int k0 = k_lo + c * KC;
+#pragma unroll
+        for (int i = 0; i < ROWS / 4; ++i) {
+            const int r = i * 4 + (lane >> 3), k = k0 + (lane & 7) * 4, n = tile * ROWS + r;
+            const bool ok = n < N && k < k_hi;
+            copy4<ALIGNED>(mine + (uint32_t)((s * STAGE + r * PITCH + (lane & 7) * 4) * 4), ok ? w + (long long)n * K + k : w, ok ? k_hi - k : 0);
+        }
+    };
+    auto copy_x = [&](int c, int s) {
+        const int k0 = k_lo + c * KC;
+#pragma unroll
+        for (int i = 0; i < (MT * 8 + 31) / 32; ++i) {
+            const int r = i * 4 + (lane >> 3), k = k0 + (lane & 7) * 4;
+            if (MT < 4 && r >= MT) continue;
+            const bool ok = r < M && k < k_hi;
+            copy4<ALIGNED>(mine + (uint32_t)((s * STAGE + ROWS * PITCH + r * KC + (lane & 7) * 4) * 4), ok ? x + (long long)r * K + k : x, ok ? k_hi - k : 0);
+        }
+    };
+    // what is asked for next: chunk `ac` of tile `at`
+    int at = blockIdx.x, ac = 0;
+    auto advance = [&]() { if (++ac == chunks) { ac = 0; at += gridDim.x; } };
+    if (chunks > 0) {
+        // the weights of the first chunks need nothing of the kernel before
+        for (int s = 0; s < STAGES - 1; ++s) {
+            if (at < n_tiles) copy_w(at, ac, s);
+            advance();
+        }
+    }
+    rdl_grid_wait();
+    rdl_grid_launch_dependents();
+    if (chunks > 0) {
+        int bt = blockIdx.x, bc = 0;
+        for (int s = 0; s < STAGES - 1; ++s) {
+            if (bt < n_tiles) copy_x(bc, s);
+            copies_commit();
+            if (++bc == chunks) { bc = 0; bt += gridDim.x; }
+        }
+    }
+    int s = 0, buf = 0;
+    for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+        unsigned long long acc[MINE];
+#pragma unroll
+        for (int m = 0; m < MINE; ++m) acc[m] = 0ull;
+        for (int c = 0; c < chunks; ++c) {
+            copies_wait<STAGES - 2>();
+            __syncwarp();                                    // chunk s is there for the whole warp, and the one before it has been read
+            const int into = s == 0 ? STAGES - 1 : s - 1;
+            if (at < n_tiles) { copy_w(at, ac, into); copy_x(ac, into); }
+            copies_commit();
+            advance();
+            const uint32_t wa = mine + (uint32_t)((s * STAGE + row * PITCH) * 4), xa = mine + (uint32_t)((s * STAGE + ROWS * PITCH + m0 * KC) * 4);
+#pragma unroll
+            for (int q = 0; q < KC / 4; ++q) {
+                const Pairs b = lds_pairs(wa + q * 16);
+#pragma unroll
+                for (int m = 0; m < MINE; ++m) {
+                    const Pairs a = lds_pairs(xa + (m * KC + q * 4) * 4);
+                    acc[m] = ffma2(a.lo, b.lo, acc[m]);
+                    acc[m] = ffma2(a.hi, b.hi, acc[m]);
+                }
+            }
+            if (++s == STAGES) s = 0;
+        }
+#pragma unroll
+        for (int m = 0; m < MINE; ++m) part[buf][warp][m0 + m][row] = halves_sum(acc[m]);
+        __syncthreads();                                     // (the other buffer was read before this barrier's predecessor was passed)
+        for (int i = threadIdx.x; i < M * ROWS; i += RUNS * 32) {
+            const int m = i / ROWS, r = i - m * ROWS, n = tile * ROWS + r;
+            float v = part[buf][0][m][r];
+#pragma unroll
+            for (int g = 1; g < RUNS; ++g) v += part[buf][g][m][r];
+            if (n < N) out[(long long)m * N + n] = v;
+        }
+        buf ^= 1;
+    }
+}
+
+constexpr int FEW_MAX = 16;
+
+template <int ROWS, int MT, bool ALIGNED>
+cudaError_t launch_few(float* out, const float* x, const float* w, int M, int N, int K, cudaStream_t st) {
+    // the ring takes what shared memory the runs' sums leave: the bytes a multiprocessor has on their way set the rate
+    constexpr int STAGE_BYTES = (ROWS * PITCH + MT * KC) * 4;
+    constexpr int FIT = (224 * 1024 - 2 * RUNS * MT * ROWS * 4) / (RUNS * STAGE_BYTES), STAGES = FIT > 10 ? 10 : FIT;
+    static_assert(STAGES >= 3, "a ring of three chunks at least");
+    constexpr size_t smem = (size_t)RUNS * STAGES * STAGE_BYTES;
+    static bool opted = false;
+    if (!opted) {
+        const cudaError_t e = cudaFuncSetAttribute(gemm_f32_few_kernel<ROWS, MT, STAGES, ALIGNED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        opted = true;
+    }
+    const int tiles = (N + ROWS - 1) / ROWS, sms = rdl_sm_count();
+    return rdl_launch(gemm_f32_few_kernel<ROWS, MT, STAGES, ALIGNED>, dim3(tiles < sms ? tiles : sms), dim3(RUNS * 32), smem, st, out, x, w, M, N, K);
+}
+
+template <bool ALIGNED>
+cudaError_t launch_few_rows(float* out, const float* x, const float* w, int M, int N, int K, cudaStream_t st) {
+    // Tiles of 16 weight rows where tiles of 32 would leave multiprocessors without one.
+    const bool narrow = (N + 31) / 32 <= rdl_sm_count();
+    if (M <= 2) return narrow ? launch_few<16, 2, ALIGNED>(out, x, w, M, N, K, st) : launch_few<32, 2, ALIGNED>(out, x, w, M, N, K, st);
+    if (M <= 4) return narrow ? launch_few<16, 4, ALIGNED>(out, x, w, M, N, K, st) : launch_few<32, 4, ALIGNED>(out, x, w, M, N, K, st);
+    if (M <= 8) return narrow ? launch_few<16, 8, ALIGNED>(out, x, w, M, N, K, st) : launch_few<32, 8, ALIGNED>(out, x, w, M, N, K, st);
+    return narrow ? launch_few<16, 16, ALIGNED>(out, x, w, M, N, K, st) : launch_few<32, 16, ALIGNED>(out, x, w, M, N, K, st);
+}
+
+// ---- many rows ----
+
+constexpr int TN = 8, BN = 16 * TN;
+// Two blocks a multiprocessor up to 64 rows a tile (hence the shorter ring there), one with 128.
+__host__ __device__ constexpr int tile_stages(int tm) { return tm == 4 ? 2 : 3; }
+
+__device__ __forceinline__ uint32_t f32_cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void f32_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float f32_ld_remote(uint32_t addr, uint32_t rank) {
+    uint32_t at;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+    return v;
+}
+
+// A tile of 16 TM rows by 128 columns; thread (ty, tx) has rows ty + 16 i and columns tx + 16 j.  SHARED: the block is one of a
+// cluster of eight along z, each with a run of k.
+template <int TM, bool SHARED, bool ALIGNED>
+__global__ void __launch_bounds__(256, TM <= 4 ? 2 : 1) gemm_f32_tile_kernel(float* __restrict__ out, const float* __restrict__ x,
+                                                                            const float* __restrict__ w, int M, int N, int K) {
+    constexpr int BM = 16 * TM, STAGE = (BM + BN) * PITCH, TILE_STAGES = tile_stages(TM);       // STAGE: floats
+    extern __shared__ __align__(16) float sm[];
+    float* sums = sm + TILE_STAGES * STAGE;                       // [BM][BN]: the runs' sums so far (SHARED: this block's run)
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tx = (lane & 7) + 8 * (warp & 1), ty = (lane >> 3) + 4 * (warp >> 1);
+    const int n0 = blockIdx.x * BN, m0 = blockIdx.y * BM;
+    const int run = run_length(K);
+    const int g_lo = SHARED ? (int)blockIdx.z : 0, g_hi = SHARED ? g_lo + 1 : RUNS;
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm);
+
+    auto copy = [&](int k, int k_hi, int s, bool weights) {      // the chunk from k on into stage s
+        if (weights) {
+#pragma unroll
+            for (int i = 0; i < BN / 32; ++i) {
+                const int r = i * 32 + (tid >> 3), kk = k + (tid & 7) * 4, n = n0 + r;
+                const bool ok = n < N && kk < k_hi;
+                copy4<ALIGNED>(base + (uint32_t)((s * STAGE + (BM + r) * PITCH + (tid & 7) * 4) * 4), ok ? w + (long long)n * K + kk : w, ok ? k_hi - kk : 0);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < (BM + 31) / 32; ++i) {
+                const int r = i * 32 + (tid >> 3), kk = k + (tid & 7) * 4, m = m0 + r;
+                if (BM % 32 && r >= BM) continue;
+                const bool ok = m < M && kk < k_hi;
+                copy4<ALIGNED>(base + (uint32_t)((s * STAGE + r * PITCH + (tid & 7) * 4) * 4), ok ? x + (long long)m * K + kk : x, ok ? k_hi - kk : 0);
+            }
+        }
+    };
+    auto run_end = [&](int g) { return min(K, (g + 1) * run); };
+    // what is asked for next: the chunk from k `ak` on of run `ag`
+    int ag = g_lo, ak = g_lo * run;
+    auto advance = [&]() { ak += KC; if (ak >= run_end(ag)) { ++ag; ak = ag * run; } };
+    auto there = [&]() { return ag < g_hi && ak < run_end(ag); };
+    for (int s = 0; s < TILE_STAGES - 1; ++s) {
+        if (there()) { copy(ak, run_end(ag), s, true); advance(); }
+    }
+    rdl_grid_wait();
+    rdl_grid_launch_dependents();
+    ag = g_lo; ak = g_lo * run;
+    for (int s = 0; s < TILE_STAGES - 1; ++s) {
+        if (there()) { copy(ak, run_end(ag), s, false); advance(); }
+        copies_commit();
+    }
+    int s = 0;
+    for (int g = g_lo; g < g_hi; ++g) {
+        unsigned long long acc[TM][TN];
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
+        for (int k = g * run; k < run_end(g); k += KC) {
+            copies_wait<TILE_STAGES - 2>();
+            __syncthreads();                                     // chunk s is there, and everybody has read the one before it
+            const int into = s == 0 ? TILE_STAGES - 1 : s - 1;
+            if (there()) { copy(ak, run_end(ag), into, true); copy(ak, run_end(ag), into, false); advance(); }
+            copies_commit();
+            const uint32_t xa = base + (uint32_t)((s * STAGE + ty * PITCH) * 4), wa = base + (uint32_t)((s * STAGE + (BM + tx) * PITCH) * 4);
+#pragma unroll 2
+            for (int q = 0; q < KC / 4; ++q) {
+                Pairs b[TN];
+#pragma unroll
+                for (int j = 0; j < TN; ++j) b[j] = lds_pairs(wa + (j * 16 * PITCH + q * 4) * 4);
+#pragma unroll
+                for (int i = 0; i < TM; ++i) {
+                    const Pairs a = lds_pairs(xa + (i * 16 * PITCH + q * 4) * 4);
+#pragma unroll
+                    for (int j = 0; j < TN; ++j) {
+                        acc[i][j] = ffma2(a.lo, b[j].lo, acc[i][j]);
+                        acc[i][j] = ffma2(a.hi, b[j].hi, acc[i][j]);
+                    }
+                }
+            }
+            if (++s == TILE_STAGES) s = 0;
+        }
+        const bool first = SHARED || g == 0, last = !SHARED && g == RUNS - 1;
+#pragma unroll
+        for (int i = 0; i < TM; ++i) {
+            const int r = ty + 16 * i;
+#pragma unroll
+            for (int j = 0; j < TN; ++j) {
+                const int c = tx + 16 * j;
+                float v = halves_sum(acc[i][j]);
+                if (!first) v = sums[r * BN + c] + v;
+                if (!last) sums[r * BN + c] = v;
+                else if (m0 + r < M && n0 + c < N) out[(long long)(m0 + r) * N + n0 + c] = v;
+            }
+        }
+    }
+    if constexpr (SHARED) {
+        f32_cluster_sync();                                      // all eight runs of the tile lie in their blocks' shared memory
+        const uint32_t rank = f32_cluster_rank();
+        const uint32_t sums_s = base + (uint32_t)(TILE_STAGES * STAGE * 4);
+        constexpr int ROWS_EACH = BM / RUNS;
+        for (int i = tid; i < ROWS_EACH * BN; i += 256) {
+            const int r = (int)rank * ROWS_EACH + i / BN, c = i % BN;
+            float v[RUNS];
+#pragma unroll
+            for (int g = 0; g < RUNS; ++g) v[g] = f32_ld_remote(sums_s + (uint32_t)((r * BN + c) * 4), g);
+#pragma unroll
+            for (int g = 1; g < RUNS; ++g) v[0] += v[g];
+            if (m0 + r < M && n0 + c < N) out[(long long)(m0 + r) * N + n0 + c] = v[0];
+        }
+        f32_cluster_sync();                                      // no block leaves while another may still read its sums
+    }
+}
+
+template <int TM, bool SHARED, bool ALIGNED>
+cudaError_t launch_tile(float* out, const float* x, const float* w, int M, int N, int K, cudaStream_t st) {
+    constexpr int BM = 16 * TM;
+    constexpr size_t smem = (size_t)(tile_stages(TM) * (BM + BN) * PITCH + BM * BN) * 4;
+    static bool opted = false;
+    if (!opted) {
+        const cudaError_t e = cudaFuncSetAttribute(gemm_f32_tile_kernel<TM, SHARED, ALIGNED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        opted = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((N + BN - 1) / BN, (M + BM - 1) / BM, SHARED ? RUNS : 1);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (SHARED) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = attr[n].val.clusterDim.y = 1;
+        attr[n++].val.clusterDim.z = RUNS;
+    }
+    if (g_rdl_programmatic_launch) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    return cudaLaunchKernelEx(&cfg, gemm_f32_tile_kernel<TM, SHARED, ALIGNED>, out, x, w, M, N, K);
+}
+
+template <int TM, bool ALIGNED>
+cudaError_t launch_tile_rows(float* out, const float* x, const float* w, int M, int N, int K, cudaStream_t st) {
+    // Eight blocks a tile where the waves of whole tiles would leave more of the chip idle than the eighths' waves do (clusters
+    // of eight reach about seven eighths of the multiprocessors, and their meeting costs about as much again).
+    const int per_sm = TM <= 4 ? 2 : 1;
+    const long long tiles = (long long)((N + BN - 1) / BN) * ((M + 16 * TM - 1) / (16 * TM));
+    const long long slots = (long long)rdl_sm_count() * per_sm, slots8 = slots * 7 / 8;
+    const double whole = (double)((tiles + slots - 1) / slots), eighths = (double)((tiles * RUNS + slots8 - 1) / slots8) / RUNS * 1.15;
+    return whole <= eighths ? launch_tile<TM, false, ALIGNED>(out, x, w, M, N, K, st) : launch_tile<TM, true, ALIGNED>(out, x, w, M, N, K, st);
+}
+
+template <bool ALIGNED>
+cudaError_t launch_rows(float* out, const float* x, const float* w, int M, int N, int K, cudaStream_t st) {
+    if (M <= FEW_MAX) return launch_few_rows<ALIGNED>(out, x, w, M, N, K, st);
+    // the tile height that pads least; from 97 rows on 128, or 64 where 128 would pad by more than a tenth
+    if (M <= 32) return launch_tile_rows<2, ALIGNED>(out, x, w, M, N, K, st);
+    if (M <= 48 || (M > 64 && M <= 96)) return launch_tile_rows<3, ALIGNED>(out, x, w, M, N, K, st);
+    const long long p128 = (M + 127) / 128 * 128LL, p64 = (M + 63) / 64 * 64LL;
+    return 10 * p128 > 11 * p64 ? launch_tile_rows<4, ALIGNED>(out, x, w, M, N, K, st) : launch_tile_rows<8, ALIGNED>(out, x, w, M, N, K, st);
 }
 
 }  // namespace
@@ -64,9 +381,10 @@ extern "C" int rdl_gemm_f32(void* out, const void* x, const void* w, int m, int 
     RDL_REQUIRE(m >= 0 && n > 0 && k > 0, "gemm_f32: bad sizes m=%d n=%d k=%d", m, n, k);
     RDL_REQUIRE(out && x && w, "gemm_f32: missing operand");
     if (m == 0) return 0;
-    dim3 grid((n + TN - 1) / TN, (m + TM - 1) / TM);
-    RDL_REQUIRE(grid.y <= 65535, "gemm_f32: %d rows exceed the grid limit", m);
-    gemm_f32_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((float*)out, (const float*)x, (const float*)w, m, n, k);
-    RDL_CHECK_LAUNCH("gemm_f32");
+    RDL_REQUIRE((m + 63) / 64 <= 65535, "gemm_f32: %d rows exceed the grid limit", m);
+    const bool aligned = k % 4 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0;
+    cudaStream_t st = (cudaStream_t)stream;
+    RDL_CHECK_EX(aligned ? launch_rows<true>((float*)out, (const float*)x, (const float*)w, m, n, k, st)
+                         : launch_rows<false>((float*)out, (const float*)x, (const float*)w, m, n, k, st), "gemm_f32");
     return 0;
 }

@@ -97,6 +97,22 @@ def test_gemm_f32_is_exact_float32(m, n, k):
     assert torch.equal(alone[0], got[m // 2])
 
 
+@pytest.mark.parametrize("k", [3, 12, 97, 100, 2304])      # a run of k shorter than four, runs that end inside a chunk, rows off 16 bytes
+def test_gemm_f32_sums_in_one_order_whatever_the_kernel(k):
+    """Few rows, every tile height and the shared tiles give the same bits for a row; operands off 16-byte boundaries too.
+    Two chains of k/16 terms and nine additions a result: (k / 16 + 9) * 2^-24 of sum |x w| bounds its error."""
+    for n in (1, 31, 130, 700):
+        x, w = rnd((300, k), torch.float32, k + n), rnd((n, k), torch.float32, n)
+        full = ops.linear(x, w)
+        bound = (x.double().abs() @ w.double().abs().t()) * (k / 16 + 9) * 2.0 ** -24
+        assert bool(((full.double() - x.double() @ w.double().t()).abs() <= bound).all())
+        for m in (1, 2, 3, 4, 5, 8, 9, 16, 17, 32, 33, 48, 49, 64, 65, 96, 97, 129, 192):
+            assert torch.equal(ops.linear(x[:m].contiguous(), w), full[:m]), (n, m)
+        off = torch.empty(n * k + 1, dtype=torch.float32, device=w.device)[1:].view(n, k).copy_(w)
+        for m in (2, 40, 300):
+            assert torch.equal(ops.linear(x[:m].contiguous(), off), full[:m]), (n, m, "off")
+
+
 def test_linear_bf16_float32_output():
     x, w = rnd((5, 96), torch.bfloat16, 11), rnd((384, 96), torch.bfloat16, 12)
     assert ops.linear(x, w, out_dtype=torch.float32).dtype is torch.float32
