@@ -1,7 +1,8 @@
-// Plain attention over new tokens and a paged cache: one warp per (query token, head),
-// float arithmetic throughout, a fixed order of operations that depends only on absolute
-// positions.  It is the attention of the 32-bit path (prefill and decode alike) and the
-// reference the fast kernels are tested against.
+// Plain attention over new tokens and a paged cache: float arithmetic throughout, a fixed order of
+// operations that depends only on absolute positions.  It is the attention of the 32-bit path (prefill
+// and decode alike) and the reference the fast kernels are tested against.  Two kernels: one warp per
+// (query token, head), any type and head size; and, for float rows that 16-byte loads can take, one block per
+// (query token, head) whose eight warps share the keys (attention_f32_kernel below).
 //
 // For query position p of a sequence and query head h (kv head g = h / (n_heads / n_kv_heads),
 // reference: rustml/core/main/src/core/tensor/ops.rs:980-987):
@@ -20,6 +21,7 @@
 // own packed key/value rows.
 #include "api.h"
 #include "common.cuh"
+#include "launch.cuh"
 
 #define PLAIN_MAX_CHUNKS 32  // head_dim <= 1024 in the wide form (the rows of a latent cache are wider than ordinary heads); 16 otherwise
 
@@ -119,6 +121,159 @@ __global__ void attention_plain_kernel(AttentionArgs a) {
     }
 }
 
+// ---------------------------------------------------------------------------------------------
+// The same for float rows whose head size is a multiple of four (up to 512): a block of eight warps per (query token, head).
+//
+// What bounds it is the latency of reading a few hundred keys; the one-warp kernel reads a key's row four bytes at a
+// time in one lane, a chain of head_dim fused multiply-adds behind each load (164 us a layer for 45 queries or 2 single
+// tokens over 40 keys of 256).  Here warp w takes the blocks of 32 absolute positions b with b mod 8 == w: eight lanes share
+// a key (16-byte loads, four keys at a time, sums by exchanges among the eight), the values are read by whole
+// warps, and the warps' sums meet in shared memory in warp order.  The order of operations depends on positions and
+// head size alone, not on the step, so logits stay bit-equal however a request is cut.
+// ---------------------------------------------------------------------------------------------
+constexpr int PF_WARPS = 8;
+
+// NC: 32-value slices of a head (head_dim <= 32 NC).
+template <int NC>
+__global__ void __launch_bounds__(PF_WARPS * 32) attention_f32_kernel(AttentionArgs a) {
+    constexpr int VC = (NC + 3) / 4;                       // 128-value slices of a head
+    __shared__ float4 part[PF_WARPS][VC][32];
+    __shared__ float part_m[PF_WARPS], part_l[PF_WARPS];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane & 7;
+    const int t = blockIdx.x, h = blockIdx.y;
+    const int hd = a.head_dim, chunks = hd / 4;            // 16-byte chunks of a row
+    const int g = h / (a.n_heads / a.n_kv_heads);
+    rdl_grid_wait();
+    rdl_grid_launch_dependents();
+    const int seq = a.tok_seq[t], p = a.tok_pos[t];
+    if (p < 0) return;  // a padding row of a fixed-size batch
+    const int cached = a.seq_cached[seq];
+    const int new_row0 = a.seq_start[seq] - a.seq_past[seq];  // packed row of position j is new_row0 + j
+    const int* table = a.tables ? a.tables + (long long)seq * a.table_width : nullptr;
+    const int lo = rdl_first_key(p, a.window, a.chunk);
+    const float* rel = a.rel_bias ? a.rel_bias + (long long)h * a.rel_len : nullptr;
+    const bool sig = a.sigmoid_bias != nullptr;
+    const float sig_bias = sig ? a.sigmoid_bias[h] : 0.f;
+    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+
+    // slice c of a lane: chunk 8 c + sub of the query
+    float4 q[NC];
+    const float4* q4 = reinterpret_cast<const float4*>((const float*)a.q + (long long)t * a.q_stride + (long long)h * hd);
+#pragma unroll
+    for (int c = 0; c < NC; ++c) q[c] = 8 * c + sub < chunks ? q4[8 * c + sub] : zero4;
+    float4 acc[VC];
+#pragma unroll
+    for (int c = 0; c < VC; ++c) acc[c] = zero4;
+    float m = -INFINITY, l = 0.f;
+
+    const int first = lo / 32, b0 = first + ((warp - first) & (PF_WARPS - 1));      // this warp's first block of positions
+    for (int b = b0; b * 32 <= p; b += PF_WARPS) {
+        // lane: where key b * 32 + lane lies (a row of the cache, stored swizzled, or a packed new row)
+        const int j = b * 32 + lane;
+        const bool valid = j >= lo && j <= p;
+        unsigned long long k_at = 0, v_at = 0;
+        int sw = -1;                                        // place of the row in its cache page; -1: a packed new row
+        if (valid) {
+            if (j < cached) {
+                const long long off = rdl_cache_offset(table, j, a.page_size, a.ring_pages, a.n_kv_heads, g, hd);
+                k_at = (unsigned long long)((const float*)a.k_cache + off);
+                v_at = (unsigned long long)((const float*)a.v_cache + off);
+                sw = j % a.page_size;
+            } else {
+                const long long off = (long long)(new_row0 + j) * a.kv_stride + (long long)g * hd;
+                k_at = (unsigned long long)((const float*)a.k_new + off);
+                v_at = (unsigned long long)((const float*)a.v_new + off);
+            }
+        }
+        // scores: four keys a pass, eight lanes a key
+        float s = 0.f;
+#pragma unroll 2
+        for (int pass = 0; pass < 8; ++pass) {
+            const int key = pass * 4 + (lane >> 3);
+            const float4* k4 = reinterpret_cast<const float4*>(__shfl_sync(0xffffffffu, k_at, key));
+            const int ksw = __shfl_sync(0xffffffffu, sw, key);
+            float4 kv[NC];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const int i = 8 * c + sub;
+                kv[c] = k4 && i < chunks ? k4[ksw < 0 ? i : rdl_swizzled_chunk(ksw, i, chunks)] : zero4;
+            }
+            float d = 0.f;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                d = fmaf(q[c].x, kv[c].x, d);
+                d = fmaf(q[c].y, kv[c].y, d);
+                d = fmaf(q[c].z, kv[c].z, d);
+                d = fmaf(q[c].w, kv[c].w, d);
+            }
+            d += __shfl_xor_sync(0xffffffffu, d, 1);
+            d += __shfl_xor_sync(0xffffffffu, d, 2);
+            d += __shfl_xor_sync(0xffffffffu, d, 4);
+            const float mine = __shfl_sync(0xffffffffu, d, (lane & 3) * 8);      // key pass * 4 + (lane & 3)
+            if ((lane >> 2) == pass) s = mine;
+        }
+        s *= a.score_scale;
+        if (a.softcap > 0.f) s = a.softcap * tanhf(s / a.softcap);
+        if (rel && valid) s += rel[min(p - j, a.rel_len - 1)];
+        float pj;
+        if (sig) {
+            pj = valid ? 1.0f / (1.0f + expf(-(s + sig_bias))) : 0.f;
+        } else {
+            const float m_new = fmaxf(m, warp_max(valid ? s : -INFINITY));
+            const float corr = m == m_new ? 1.f : expf(m - m_new);                // exp(-inf) = 0 on the first block
+            pj = !valid || s == -INFINITY ? 0.f : expf(s - m_new);
+            l = l * corr + warp_sum(pj);
+            m = m_new;
+#pragma unroll
+            for (int c = 0; c < VC; ++c) { acc[c].x *= corr; acc[c].y *= corr; acc[c].z *= corr; acc[c].w *= corr; }
+        }
+        const int j0 = max(lo - b * 32, 0), j1 = min(p - b * 32, 31);
+#pragma unroll 8
+        for (int jj = j0; jj <= j1; ++jj) {
+            const float pw = __shfl_sync(0xffffffffu, pj, jj);
+            const float4* v4 = reinterpret_cast<const float4*>(__shfl_sync(0xffffffffu, v_at, jj));
+            const int vsw = __shfl_sync(0xffffffffu, sw, jj);
+#pragma unroll
+            for (int c = 0; c < VC; ++c) {
+                const int i = 32 * c + lane;
+                const float4 v = i < chunks ? v4[vsw < 0 ? i : rdl_swizzled_chunk(vsw, i, chunks)] : zero4;
+                acc[c].x = fmaf(pw, v.x, acc[c].x);
+                acc[c].y = fmaf(pw, v.y, acc[c].y);
+                acc[c].z = fmaf(pw, v.z, acc[c].z);
+                acc[c].w = fmaf(pw, v.w, acc[c].w);
+            }
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < VC; ++c) part[warp][c][lane] = acc[c];
+    if (lane == 0) { part_m[warp] = m; part_l[warp] = l; }
+    __syncthreads();
+    // the warps' sums, in warp order; the sink joins the denominator once, neither scaled nor capped
+    float m_all = a.sinks ? a.sinks[h] : -INFINITY;
+#pragma unroll
+    for (int w = 0; w < PF_WARPS; ++w) m_all = fmaxf(m_all, part_m[w]);
+    float f[PF_WARPS], l_all = 0.f;
+#pragma unroll
+    for (int w = 0; w < PF_WARPS; ++w) {
+        f[w] = sig ? 1.f : (part_m[w] == m_all ? 1.f : expf(part_m[w] - m_all));
+        l_all += part_l[w] * f[w];
+    }
+    if (a.sinks) l_all += expf(a.sinks[h] - m_all);
+    const float inv = sig ? 1.0f : 1.0f / l_all;
+    float* o = (float*)a.out + (long long)t * a.out_stride + (long long)h * hd;
+    for (int i = threadIdx.x; i < hd; i += PF_WARPS * 32) {
+        float v = 0.f;
+#pragma unroll
+        for (int w = 0; w < PF_WARPS; ++w) v = fmaf(reinterpret_cast<const float*>(part[w])[i], f[w], v);
+        o[i] = v * inv;
+    }
+}
+
+template <int NC>
+static cudaError_t launch_attention_f32(const AttentionArgs& a, cudaStream_t st) {
+    return rdl_launch(attention_f32_kernel<NC>, dim3(a.n_tokens, a.n_heads), dim3(PF_WARPS * 32), 0, st, a);
+}
+
 int rdl_check_attention_args(const AttentionArgs* a, const char* who) {
     RDL_REQUIRE(rdl_valid_dtype(a->dtype), "%s: bad dtype %d", who, a->dtype);
     RDL_REQUIRE(a->n_tokens >= 0 && a->n_seqs >= 0, "%s: bad token or sequence count", who);
@@ -146,6 +301,16 @@ extern "C" int rdl_attention_plain(const AttentionArgs* a, void* stream) {
     if (int e = rdl_check_attention_args(a, "attention_plain")) return e;
     RDL_REQUIRE(a->head_dim <= 32 * PLAIN_MAX_CHUNKS, "attention_plain: head_dim %d exceeds %d", a->head_dim, 32 * PLAIN_MAX_CHUNKS);
     if (a->n_tokens == 0) return 0;
+    // 16-byte loads: whole rows of chunks, on 16-byte boundaries (the choice rests on the model's layout, not on the step)
+    auto quads = [](const void* p, long long stride) { return (uintptr_t)p % 16 == 0 && stride % 4 == 0; };
+    if (a->dtype == RDL_F32 && a->head_dim % 4 == 0 && a->head_dim <= 512 && a->n_heads <= 65535 && quads(a->q, a->q_stride) &&
+        (!a->tables || (quads(a->k_cache, 0) && quads(a->v_cache, 0))) && (!a->k_new || (quads(a->k_new, a->kv_stride) && quads(a->v_new, a->kv_stride)))) {
+        cudaStream_t st = (cudaStream_t)stream;
+        const int hd = a->head_dim;
+        RDL_CHECK_EX(hd <= 32 ? launch_attention_f32<1>(*a, st) : hd <= 64 ? launch_attention_f32<2>(*a, st) : hd <= 128 ? launch_attention_f32<4>(*a, st)
+                     : hd <= 256 ? launch_attention_f32<8>(*a, st) : launch_attention_f32<16>(*a, st), "attention_plain");
+        return 0;
+    }
     const int warps = 4;
     const long long items = (long long)a->n_tokens * a->n_heads;
     const unsigned blocks = (unsigned)((items + warps - 1) / warps);

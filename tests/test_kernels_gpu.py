@@ -363,6 +363,19 @@ def test_attention_over_cache_and_new_rows(shape, dtype, kind):
         assert_close(got, want, dtype, rel=6.0, what=f"{kind} softcap={softcap}")
 
 
+@pytest.mark.parametrize("shape", [
+    dict(past=[700, 0, 31], new=[1, 300, 2], n_heads=4, n_kv_heads=2, head_dim=512, page_size=64, window=None),   # several blocks of keys a warp
+    dict(past=[520, 255], new=[3, 1], n_heads=3, n_kv_heads=1, head_dim=36, page_size=16, window=270),            # a first block cut by the window
+    dict(past=[40], new=[2], n_heads=2, n_kv_heads=2, head_dim=10, page_size=16, window=None),                    # rows that are not 16-byte chunks
+])
+def test_float32_attention_shares_the_keys_among_warps(shape):
+    c = Case(dtype=torch.float32, seed=33, **shape)
+    b = c.batch("past")
+    got = ops.attention(c.qkv, b, c.pages, new_kv=c.new_kv(), kind="plain", **c.kw(softcap=5.0))
+    want = ref.attention(c.qkv, b, c.pages, new_kv=c.new_kv(), **c.kw(softcap=5.0))
+    assert_close(got, want, torch.float32, what="float32 attention", f32_tol=c.max_total * 2.0 ** -24)     # sums over the keys
+
+
 TC_SHAPES = [
     dict(new=[1], n_heads=1, n_kv_heads=1, head_dim=64, window=None),
     dict(new=[5, 129, 70], n_heads=4, n_kv_heads=2, head_dim=64, window=None),
