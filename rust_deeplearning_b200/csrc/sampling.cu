@@ -257,8 +257,15 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(int* __restrict_
 // the run or on the batch.  Same order of operations and same meaning of the options as above.  Measured at
 // 256,000 tokens, one row: 34 us plain, 92 us with top-k or top-p, 151 us with both (118 / 606 / 887 / 1,289 us
 // in the one-block kernel); two bits a round (three nested candidates) was no faster.
+//
+// With a top-k of up to FEW_TOP_K the rounds are not needed (few_candidates below): the k-th largest of a block's 1,024
+// largest-of-a-thread values is a bound that at least k elements reach and that few others do, so the elements at or above
+// the highest block's bound - a few dozen of 256,000 - go to one block, which sorts them and does the rest alone.  What
+// bounds it is the row's one trip from L2 and two cluster barriers.  Rows with more candidates than a block sorts (long ties), with fewer
+// than k numbers above minus infinity, or with an infinity or NaN at the top take the rounds.
 // ---------------------------------------------------------------------------------------------
 constexpr int CL_THREADS = 1024, CL_ITEMS = 32, CL_PER_BLOCK = CL_THREADS * CL_ITEMS, CL_MAX_BLOCKS = 8;
+constexpr int FEW_TOP_K = 256, FEW_CAP = CL_THREADS;      // candidates one block sorts, a thread each
 
 __device__ __forceinline__ uint32_t cl_rank() {
     uint32_t r;
@@ -391,6 +398,181 @@ __global__ void __launch_bounds__(CL_THREADS, 1) argmax_cluster_kernel(int* __re
     cl_sync();                 // no block leaves while the first may still read its shared memory
 }
 
+// The float an ordered key came from.
+__device__ __forceinline__ float key_value(unsigned key) {
+    return __uint_as_float((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key);
+}
+
+// Warp 0: the first place of `mass[0 .. n)` at which the running sum passes `target` (strictly, or reaches it), n if none does;
+// total: the whole sum.  The sums are formed 32 at a time, in the order of a doubling scan.
+__device__ __forceinline__ int first_beyond(const float* mass, int n, float target, bool strictly, float& total) {
+    const int lane = threadIdx.x & 31;
+    float carry = 0.f;
+    int found = n;
+    for (int b = 0; b < n; b += 32) {
+        float v = b + lane < n ? mass[b + lane] : 0.f;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float up = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += up;
+        }
+        v += carry;
+        const unsigned hit = __ballot_sync(0xffffffffu, b + lane < n && (strictly ? v > target : v >= target));
+        if (hit && found == n) found = b + __ffs(hit) - 1;
+        carry = __shfl_sync(0xffffffffu, v, 31);
+    }
+    total = carry;
+    return found;
+}
+
+// Top-k of up to FEW_TOP_K (see above).  false, the same in every block of the cluster: the row is not one for it, nothing was
+// written.  `list`: at least 6 * FEW_CAP words of shared memory.
+__device__ __noinline__ bool few_candidates(int* out_tokens, int* host_tokens, const float* src, int row, int vocab, const SamplingArgs& prm,
+                               const unsigned long long* row_stream, const int* row_step, int rank, int n_blocks, unsigned* list,
+                               ClusterExchange* x, int& parity) {
+    __shared__ int n_mine, keep_k;
+    const int tid = threadIdx.x;
+    const int base = rank * CL_PER_BLOCK + 4 * tid;        // the thread's elements: groups of four, 4 * CL_THREADS apart
+    float v[CL_ITEMS];
+    if (vocab % 4 == 0 && (uintptr_t)src % 16 == 0) {
+#pragma unroll
+        for (int u = 0; u < CL_ITEMS / 4; ++u) {
+            const int at = base + 4 * CL_THREADS * u;
+            const float4 q = at < vocab ? __ldcg(reinterpret_cast<const float4*>(src + at)) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+            v[4 * u] = q.x; v[4 * u + 1] = q.y; v[4 * u + 2] = q.z; v[4 * u + 3] = q.w;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < CL_ITEMS; ++i) {
+            const int at = base + 4 * CL_THREADS * (i >> 2) + (i & 3);
+            v[i] = at < vocab ? __ldcg(src + at) : -INFINITY;
+        }
+    }
+    // dividing by the temperature keeps the order, so only the thread's largest is divided here
+    unsigned best = 0u;
+#pragma unroll
+    for (int i = 0; i < CL_ITEMS; ++i) best = max(best, ordered_key(v[i]));
+    const bool at_top = best >= 0xff800000u;               // an infinity or a NaN
+    best = ordered_key(key_value(best) / prm.temperature);
+    // A bound that k of the block's 1,024 largest-of-a-thread keys reach, and not many more: bit by bit from the top, until
+    // the count is close enough.
+    unsigned bound = 0u;
+    for (int bit = 31; bit >= 0; --bit) {
+        const unsigned cand = bound | (1u << bit);
+        const int c = __syncthreads_count(best >= cand);
+        if (c >= prm.top_k) {
+            bound = cand;
+            if (c <= prm.top_k + 24) break;
+        }
+    }
+    if (tid == 0) { x->u[parity] = bound; n_mine = 0; }
+    cl_sync();
+    for (int r = 0; r < n_blocks; ++r) bound = max(bound, cl_ld_u32(cl_map(&x->u[parity], r)));
+    parity ^= 1;
+    if (best >= bound) {
+        if (at_top) atomicAdd(&n_mine, FEW_CAP + 1);
+        // what is below this before the division is below the bound after it
+        const float scaled = key_value(bound) * prm.temperature, maybe = scaled - fabsf(scaled) * 1e-5f - 1e-37f;
+#pragma unroll
+        for (int i = 0; i < CL_ITEMS; ++i) {
+            if (!(v[i] >= maybe)) continue;
+            const unsigned key = ordered_key(v[i] / prm.temperature);
+            if (key < bound) continue;
+            const int p = atomicAdd(&n_mine, 1);
+            if (p < FEW_CAP) { list[p] = key; list[FEW_CAP + p] = (unsigned)(base + 4 * CL_THREADS * (i >> 2) + (i & 3)); }
+        }
+    }
+    __syncthreads();
+    cl_sync();                                             // every block's candidates lie in its shared memory
+    unsigned n = 0u, from = 0u;
+    for (int r = 0; r < n_blocks; ++r) n += cl_ld_u32(cl_map(&n_mine, r));
+    const bool few = bound > ordered_key(-INFINITY) && n <= (unsigned)FEW_CAP;
+    unsigned* all_key = list + 2 * FEW_CAP;
+    unsigned* all_idx = all_key + FEW_CAP;
+    if (few && rank == 0) {
+        for (int r = 0; r < n_blocks; ++r) {
+            const unsigned c = cl_ld_u32(cl_map(&n_mine, r));
+            if (tid < (int)c) {
+                all_key[from + tid] = cl_ld_u32(cl_map(list + tid, r));
+                all_idx[from + tid] = cl_ld_u32(cl_map(list + FEW_CAP + tid, r));
+            }
+            from += c;
+        }
+    }
+    __syncthreads();
+    cl_sync();                                             // the first block has them; the others are done
+    if (!few) return false;
+    if (rank != 0) return true;
+    // The k-th largest of them (eight blocks bring about eight times k), again bit by bit, and those that are as large: ties are kept.
+    unsigned my_key = tid < (int)n ? all_key[tid] : 0u, my_idx = tid < (int)n ? all_idx[tid] : 0u, kth = 0u;
+    for (int bit = 31; bit >= 0; --bit) {
+        const unsigned cand = kth | (1u << bit);
+        const int c = __syncthreads_count(my_key >= cand);
+        if (c >= prm.top_k) {
+            kth = cand;
+            if (c == prm.top_k) break;
+        }
+    }
+    if (tid == 0) n_mine = 0;
+    const int n_k = __syncthreads_count(my_key >= kth);    // (kth > 0, and 0 stands for "not there")
+    if (my_key >= kth) {
+        const int p = atomicAdd(&n_mine, 1);
+        list[p] = my_key;                                  // (the first block's own list is read no more)
+        list[FEW_CAP + p] = my_idx;
+    }
+    __syncthreads();
+    // sorted: larger keys first, smaller indices first among equal ones
+    unsigned* sort_key = all_key;
+    unsigned* sort_idx = all_idx;
+    if (tid < n_k) {
+        my_key = list[tid];
+        my_idx = list[FEW_CAP + tid];
+        int place = 0;
+#pragma unroll 4
+        for (int i = 0; i < n_k; ++i) {
+            const unsigned k = list[i];
+            place += k > my_key || (k == my_key && list[FEW_CAP + i] < my_idx);
+        }
+        sort_key[place] = my_key;
+        sort_idx[place] = my_idx;
+    }
+    float* mass = reinterpret_cast<float*>(list + 4 * FEW_CAP);
+    unsigned* drawn_idx = list + 5 * FEW_CAP;
+    __syncthreads();
+    if (tid < n_k) { my_key = sort_key[tid]; my_idx = sort_idx[tid]; }
+    const float mx = key_value(sort_key[0]);
+    const float e = tid < n_k ? expf(key_value(my_key) - mx) : 0.f;
+    mass[tid] = e;
+    __syncthreads();
+    if (prm.top_p < 1.0f && tid < 32) {
+        float z, again;
+        first_beyond(mass, n_k, INFINITY, true, z);
+        const int at = first_beyond(mass, n_k, prm.top_p * z, false, again);
+        if (tid == 0) keep_k = at < n_k ? at : n_k - 1;
+    }
+    __syncthreads();
+    int n_p = n_k;
+    if (prm.top_p < 1.0f) n_p = __syncthreads_count(tid < n_k && my_key >= sort_key[keep_k]);      // ties with the last one are kept
+    // the draw goes by index
+    if (tid < n_p) {
+        int place = 0;
+#pragma unroll 4
+        for (int i = 0; i < n_p; ++i) place += sort_idx[i] < my_idx;
+        mass[place] = e;                                   // (read for the last time before the barrier above)
+        drawn_idx[place] = my_idx;
+    }
+    __syncthreads();
+    if (tid < 32) {
+        float total, again;
+        first_beyond(mass, n_p, INFINITY, true, total);
+        const float u = uniform_from(prm.seed, row_stream ? row_stream[row] : (unsigned long long)row,
+                                     row_step ? (unsigned long long)row_step[row] : 0ull);
+        const int at = first_beyond(mass, n_p, u * total, true, again);
+        if (tid == 0) put_token(out_tokens, host_tokens, row, (int)drawn_idx[at < n_p ? at : n_p - 1]);
+    }
+    return true;
+}
+
 __global__ void __launch_bounds__(CL_THREADS, 1) sample_cluster_kernel(int* __restrict__ out_tokens, int* __restrict__ host_tokens, const float* __restrict__ logits,
                                                                        int vocab, SamplingArgs prm,
                                                                        const unsigned long long* __restrict__ row_stream,
@@ -433,6 +615,9 @@ __global__ void __launch_bounds__(CL_THREADS, 1) sample_cluster_kernel(int* __re
         cl_sync();
         src = w;
     }
+    if (prm.top_k > 0 && prm.top_k < vocab && prm.top_k <= FEW_TOP_K &&
+        few_candidates(out_tokens, host_tokens, src, row, vocab, prm, row_stream, row_step, rank, n_blocks, keys, &xch, parity))
+        return;
     float e[CL_ITEMS];                                        // the scaled logits first, their exponentials later
     float mx = -INFINITY;
 #pragma unroll

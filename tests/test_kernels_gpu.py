@@ -583,6 +583,25 @@ def test_sampling(vocab):
             assert got == want, (kw, step, got, want)
 
 
+@pytest.mark.parametrize("vocab", [300, 32768, 65538, 131072])
+def test_sampling_of_few_candidates_and_rows_that_have_more(vocab):
+    """Top-k up to 256 (a block sorts the candidates) and above; rows with long ties at the k-th value, with fewer finite
+    logits than k, and with equal candidates in different blocks."""
+    rows = 6
+    logits = rnd((rows, vocab), torch.float32, 61, 2.0)
+    logits[1] = torch.round(logits[1])                                # long ties at every value
+    logits[2, 40:] = -math.inf                                        # 40 finite ones
+    logits[3, :: max(vocab // 9, 1)] = 20.0                           # equal maxima spread over the row
+    logits[4] = logits[4].clamp(max=1.0)                              # the maximum is a long tie
+    logits[5, vocab - 1] = 30.0
+    stream = torch.arange(rows, dtype=torch.int64, device=DEV) + 3
+    steps = torch.full((rows,), 2, dtype=torch.int32, device=DEV)
+    for top_k in (1, 2, 40, 255, 256, 257):
+        for top_p in (1.0, 0.5, 0.97):
+            args = dict(temperature=0.9, seed=5, row_stream=stream, row_step=steps, top_k=top_k, top_p=top_p)
+            assert ops.sample(logits, **args).tolist() == ref.sample(logits, **args).tolist(), (top_k, top_p)
+
+
 @pytest.mark.parametrize("vocab", [256, 40000])
 def test_sampling_takes_minus_zero_for_zero(vocab):
     """Logits that are +0 and -0 in turn are all equal: the thresholds of top-k and top-p (found on bit patterns)
