@@ -20,8 +20,12 @@
 
 __device__ __forceinline__ float silu_f(float z) { return z / (1.0f + expf(-z)); }
 
+// A single-token step is bound by the state's way in and out, that is by the blocks a multiprocessor holds and by how
+// soon each asks for its part: left alone the compiler took 128 registers (two blocks a multiprocessor), and the state
+// was asked for behind four trips to memory in a row.  Four blocks (64 registers), everything
+// that hangs on the sequence alone asked for at once: 32 sequences of 16 heads of 128 x 128 (67 MB): 23.9 -> 21.0 us.
 template <typename T, int RPT>
-__global__ void __launch_bounds__(256) decay_scan_kernel(DecayAttentionArgs a) {
+__global__ void __launch_bounds__(256, RPT <= 8 ? 5 : (RPT == 16 ? 4 : (RPT == 32 ? 2 : 1))) decay_scan_kernel(DecayAttentionArgs a) {
     extern __shared__ float sm[];
     const int dim = a.dim, vdim = a.vdim;
     float* q_raw = sm;                       // [2][dim]
@@ -33,15 +37,15 @@ __global__ void __launch_bounds__(256) decay_scan_kernel(DecayAttentionArgs a) {
     rdl_grid_wait();
     rdl_grid_launch_dependents();
     const int seq = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * DA_COLS;
-    const int row0 = a.seq_start[seq], n = a.seq_start[seq + 1] - row0;
+    const int row0 = a.seq_start[seq], n = a.seq_start[seq + 1] - row0, slot = a.slots[seq];
     if (n <= 0) return;
-    if (a.tok_pos[row0] < 0) return;         // a padding sequence of a fixed-size batch
+    const int first_pos = a.tok_pos[row0];   // (negative: a padding sequence of a fixed-size batch, which left its slot's state alone)
     const int tid = threadIdx.x, j = tid & 31, r = tid >> 5, n_thr = blockDim.x;
     const int col = c0 + j;
     const bool col_ok = col < vdim;
     const int i0 = r * RPT;
     const float decay = a.decay[h];
-    float* S = a.state + (((long long)a.slots[seq] * a.n_heads + h) * dim) * vdim;
+    float* S = a.state + (((long long)slot * a.n_heads + h) * dim) * vdim;
     float s_reg[RPT];
 #pragma unroll
     for (int i = 0; i < RPT; ++i) s_reg[i] = (col_ok && i0 + i < dim) ? S[(long long)(i0 + i) * vdim + col] : 0.f;
@@ -68,13 +72,14 @@ __global__ void __launch_bounds__(256) decay_scan_kernel(DecayAttentionArgs a) {
         if (r == 0) v_in[b * DA_COLS + j] = a.silu ? silu_f(pv) : pv;
     };
     fetch(0);
+    if (first_pos < 0) return;
     stage(0);
     __syncthreads();
     for (int t = 0; t < n; ++t) {
         const int b = t & 1;
         if (t + 1 < n) fetch(t + 1);
         // q and k of this token as they enter the recurrence
-        const int pos = a.tok_pos[row0 + t];
+        const int pos = t == 0 ? first_pos : a.tok_pos[row0 + t];
         for (int i = tid; i < dim; i += n_thr) {
             float qv, kv;
             if (i < 2 * half) {

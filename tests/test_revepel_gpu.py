@@ -92,6 +92,14 @@ def test_norm_and_token_shift(dtype, width, lens, past):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("width", [4, 30, 260, 2048, 8192, 8196])
+def test_norm_and_token_shift_at_every_depth(dtype, width):
+    """Rows held in registers at each depth (one group of four values a thread up to eight), and the widths beside them
+    that are no multiple of four or too wide."""
+    test_norm_and_token_shift(dtype, width, [1, 3, 1, 2], [6, 0, 0, 2])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("taps,channels,lens,past,bias", [(4, 40, [9, 1, 2, 1], [0, 5, 0, 0], True), (2, 130, [3, 30], [1, 0], False),
                                                           (1, 24, [4], [2], True), (3, 300, [1, 2, 70], [1, 1, 2], False), (8, 16, [3, 20], [0, 4], True)])
 def test_short_convolution_with_carried_inputs(dtype, taps, channels, lens, past, bias):
