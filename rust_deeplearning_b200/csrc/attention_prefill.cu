@@ -7,6 +7,13 @@
 // 64 positions aligned to absolute multiples of 64; tiles wholly outside the window are skipped.
 // Products run on the tensor cores (mma.sync m16n8k16, float accumulators); scores, tanh,
 // exponentials, row maxima and row sums are float.
+//
+// A few new tokens behind a long past (a conversation's next turn) make few blocks with many keys each: 3 x 41 tokens of 8
+// heads are 24 blocks that walk 640 to 720 keys one tile after the other, 160 us.  There a cluster of up to eight blocks
+// takes a query tile and head, each a run of its key tiles; every block leaves its unnormalised sums, maxima and normalisers
+// in its shared memory, and each merges its share of the rows in the order of the runs.  The host takes the largest of
+// 2, 4, 8 with which the blocks still find room at once; the place of a tile's page is looked up once a tile and not once
+// a row and chunk.  Together 160 -> 32 us.
 #include "api.h"
 #include "common.cuh"
 #include "launch.cuh"
@@ -50,9 +57,28 @@ __device__ __forceinline__ uint32_t tile_addr(uint32_t base, int row, int chunk)
     return base + (uint32_t)((row * (HD / 8) + swizzled_chunk<HD>(row, chunk)) * 16);
 }
 
+__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// what block `rank` of the cluster has at this block's shared address `addr`
+__device__ __forceinline__ float ld_block(uint32_t addr, uint32_t rank) {
+    float v;
+    asm volatile("{\n.reg .b32 a;\nmapa.shared::cluster.u32 a, %1, %2;\nld.shared::cluster.f32 %0, [a];\n}" : "=f"(v) : "r"(addr), "r"(rank) : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 ld_block4(uint32_t addr, uint32_t rank) {
+    float4 v;
+    asm volatile("{\n.reg .b32 a;\nmapa.shared::cluster.u32 a, %4, %5;\nld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [a];\n}"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr), "r"(rank) : "memory");
+    return v;
+}
+
+constexpr int MAX_RUNS = 8;
+
 // MODE 0: softmax; 1: sigmoid weights; 2: softmax with a bias per head and distance (base-2 domain) added to the scores
 template <int HD, int MODE>
-__global__ void __launch_bounds__(NTHREADS) attention_prefill_kernel(AttentionArgs a) {
+__global__ void __launch_bounds__(NTHREADS) attention_prefill_kernel(AttentionArgs a, int runs) {
     constexpr int CH = HD / 8;          // 16-byte chunks per row
     extern __shared__ __align__(128) unsigned char smem[];
     const uint32_t sQ = (uint32_t)__cvta_generic_to_shared(smem);
@@ -60,7 +86,8 @@ __global__ void __launch_bounds__(NTHREADS) attention_prefill_kernel(AttentionAr
     const uint32_t sV = sK + BN * HD * 2;
     unsigned char* gQ = smem;
 
-    const int tile = a.n_tiles - 1 - blockIdx.x, h = blockIdx.y;   // later tiles of a sequence have more keys: start them first
+    const int run = runs > 1 ? (int)cluster_rank() : 0;
+    const int tile = a.n_tiles - 1 - (int)blockIdx.x / runs, h = blockIdx.y;   // later tiles of a sequence have more keys: start them first
     const int seq = a.tile_seq[tile], q0 = a.tile_q0[tile];
     const int row0 = a.seq_start[seq];
     const int n_new = a.seq_start[seq + 1] - row0;
@@ -112,10 +139,15 @@ __global__ void __launch_bounds__(NTHREADS) attention_prefill_kernel(AttentionAr
     // One tile of keys (which == 0) or values (which == 1) on its way to shared memory: asynchronous
     // 16-byte copies that bypass the registers, rows beyond the sequence and chunks beyond head_dim
     // filled with zeros.  Each call is one commit group.
+    const bool whole_pages = a.page_size % BN == 0;
     auto issue = [&](int kv0, int which) {
         const uint32_t sdst = which ? sV : sK;
         const __nv_bfloat16* cache_base = which ? vcache : kcache;
         const __nv_bfloat16* new_base = which ? vnew : knew;
+        // a tile that lies in one page: the page is looked up once
+        const __nv_bfloat16* page = nullptr;
+        if (whole_pages && kv0 < cached) page = cache_base + rdl_cache_offset(table, kv0, a.page_size, a.ring_pages, a.n_kv_heads, g, hd);
+#pragma unroll 4
         for (int idx = tid; idx < BN * CH; idx += NTHREADS) {
             const int r = idx / CH, c = idx - r * CH;
             const int j = kv0 + r;
@@ -124,7 +156,7 @@ __global__ void __launch_bounds__(NTHREADS) attention_prefill_kernel(AttentionAr
             if (j <= p_last && c * 8 < hd) {
                 bytes = 16;
                 if (j < cached)   // chunks of a cache row are stored swizzled by the row's place in its page
-                    src = cache_base + rdl_cache_offset(table, j, a.page_size, a.ring_pages, a.n_kv_heads, g, hd) +
+                    src = whole_pages ? page + (long long)r * hd + rdl_swizzled_chunk(r, c, hd / 8) * 8 : cache_base + rdl_cache_offset(table, j, a.page_size, a.ring_pages, a.n_kv_heads, g, hd) +
                           rdl_swizzled_chunk(j % a.page_size, c, hd / 8) * 8;
                 else
                     src = new_base + (long long)(row0 + j - past) * a.kv_stride + (long long)g * hd + c * 8;
@@ -134,13 +166,18 @@ __global__ void __launch_bounds__(NTHREADS) attention_prefill_kernel(AttentionAr
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
 
-    const int kv_first = (lo_first / BN) * BN;
-    if (kv_first <= p_last) {
+    int kv_first = (lo_first / BN) * BN, kv_end = p_last + 1;       // this block's keys: whole tiles of the query tile's
+    if (runs > 1) {
+        const int n_kt = (p_last - kv_first) / BN + 1, first = kv_first;
+        kv_first = first + run * n_kt / runs * BN;
+        kv_end = min(first + (run + 1) * n_kt / runs * BN, kv_end);
+    }
+    if (kv_first < kv_end) {
         issue(kv_first, 0);
         issue(kv_first, 1);
     }
-    for (int kv0 = kv_first; kv0 <= p_last; kv0 += BN) {
-        const bool has_next = kv0 + BN <= p_last;
+    for (int kv0 = kv_first; kv0 < kv_end; kv0 += BN) {
+        const bool has_next = kv0 + BN < kv_end;
         asm volatile("cp.async.wait_group 1;\n" ::: "memory");   // this tile's keys have landed (its values may be on the way)
         __syncthreads();
 
@@ -265,6 +302,75 @@ __global__ void __launch_bounds__(NTHREADS) attention_prefill_kernel(AttentionAr
         if (has_next) issue(kv0 + BN, 1);      // the next values travel while the next scores are computed
     }
 
+    if (runs > 1) {
+        // ---- the cluster's blocks meet: [64 rows][HD + 4] sums, then maxima, then normalisers, where the tiles lay ----
+        constexpr int PITCH = HD + 4;
+        const uint32_t sums = sQ, stats = sQ + BM * PITCH * 4;
+        static_assert(BM * PITCH * 4 + 2 * BM * 4 <= (BM + 2 * BN) * HD * 2, "the merge fits where the tiles lay");
+        __shared__ float weight_s[BM / 2][MAX_RUNS], inv_s[BM / 2];
+        float* so = reinterpret_cast<float*>(smem);
+        float* st = so + BM * PITCH;
+        const int w0 = warp * 16 + quad, w1 = w0 + 8;
+        __syncthreads();                   // (a block without keys has not waited for the others' query tile yet)
+#pragma unroll
+        for (int nt = 0; nt < HD / 8; ++nt) {
+            *reinterpret_cast<float2*>(so + w0 * PITCH + nt * 8 + 2 * tq) = make_float2(o[nt][0], o[nt][1]);
+            *reinterpret_cast<float2*>(so + w1 * PITCH + nt * 8 + 2 * tq) = make_float2(o[nt][2], o[nt][3]);
+        }
+        if (tq == 0) { st[w0] = m0; st[w1] = m1; st[BM + w0] = l0; st[BM + w1] = l1; }
+        __syncwarp();
+        cluster_sync();
+        const int share = BM / runs, first_row = run * share;
+        if (tid < share) {
+            const int r = first_row + tid;
+            float M = -INFINITY, L = 0.f, m[MAX_RUNS], l[MAX_RUNS];
+#pragma unroll
+            for (int s = 0; s < MAX_RUNS; ++s) {
+                if (s < runs) {
+                    m[s] = ld_block(stats + (uint32_t)(r * 4), (uint32_t)s);
+                    l[s] = ld_block(stats + (uint32_t)((BM + r) * 4), (uint32_t)s);
+                    M = fmaxf(M, m[s]);
+                }
+            }
+#pragma unroll
+            for (int s = 0; s < MAX_RUNS; ++s) {
+                if (s < runs) {
+                    const float w = sig ? 1.0f : (m[s] == -INFINITY ? 0.f : exp2f(m[s] - M));      // (sigmoid weights are not rescaled)
+                    weight_s[tid][s] = w;
+                    L = fmaf(w, l[s], L);
+                }
+            }
+            if (a.sinks) L += exp2f(a.sinks[h] * LOG2E - M);
+            inv_s[tid] = sig ? 1.0f : 1.0f / L;
+        }
+        __syncthreads();
+        __nv_bfloat16* out = (__nv_bfloat16*)a.out;
+        const int quads = hd / 4;
+        for (int idx = tid; idx < share * quads; idx += NTHREADS) {
+            const int i = idx / quads, d = (idx - i * quads) * 4, r = first_row + i;
+            if (r >= rows) continue;
+            float4 part[MAX_RUNS];
+#pragma unroll
+            for (int s = 0; s < MAX_RUNS; ++s)
+                if (s < runs) part[s] = ld_block4(sums + (uint32_t)((r * PITCH + d) * 4), (uint32_t)s);
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int s = 0; s < MAX_RUNS; ++s) {
+                if (s < runs) {
+                    const float w = weight_s[i][s];
+                    acc.x = fmaf(w, part[s].x, acc.x); acc.y = fmaf(w, part[s].y, acc.y);
+                    acc.z = fmaf(w, part[s].z, acc.z); acc.w = fmaf(w, part[s].w, acc.w);
+                }
+            }
+            const float inv = inv_s[i];
+            __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(out + (long long)(row0 + q0 + r) * a.out_stride + (long long)h * hd + d);
+            o2[0] = __floats2bfloat162_rn(acc.x * inv, acc.y * inv);
+            o2[1] = __floats2bfloat162_rn(acc.z * inv, acc.w * inv);
+        }
+        __syncwarp();
+        cluster_sync();                    // the others may still read this block's sums
+        return;
+    }
     // ---- normalise and store ----
     const int r0 = warp * 16 + quad, r1 = r0 + 8;
     if (a.sinks) {      // a logit without key or value joins each row's denominator (base-2 domain, like m and l)
@@ -292,13 +398,32 @@ template <int HD, int MODE>
 int launch_prefill_as(const AttentionArgs* a, cudaStream_t st) {
     const int smem = (BM + 2 * BN) * HD * 2;
     static bool opted = false;
-    if (smem > 48 * 1024 && !opted) {
+    if (smem > 40 * 1024 && !opted) {      // (the kernel has a little static shared memory too)
         RDL_CUDA(cudaFuncSetAttribute(attention_prefill_kernel<HD, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
                  "attention_prefill");
         opted = true;
     }
-    dim3 grid(a->n_tiles, a->n_heads);
-    RDL_CHECK_EX(rdl_launch(attention_prefill_kernel<HD, MODE>, grid, dim3(NTHREADS), (size_t)smem, st, *a), "attention_prefill");
+    // Runs of keys: none where the query tiles alone fill the chip, else the most with which all blocks find room at once
+    // (two a multiprocessor for the widest heads).  How many keys there are is known on the device only; runs without keys
+    // cost their part of the merge (about 3 us).
+    const long long blocks = (long long)a->n_tiles * a->n_heads;
+    int runs = 1;
+    while (runs < MAX_RUNS && blocks * 2 * runs <= 2LL * rdl_sm_count()) runs *= 2;
+    RDL_REQUIRE(blocks * runs <= 0x7fffffffLL, "attention_prefill: too many query tiles for one grid");
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)runs;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3((unsigned)(a->n_tiles * runs), (unsigned)a->n_heads);
+    cfg.blockDim = dim3(NTHREADS);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_rdl_programmatic_launch ? 2 : 1;
+    RDL_CHECK_EX(cudaLaunchKernelEx(&cfg, attention_prefill_kernel<HD, MODE>, *a, runs), "attention_prefill");
     return 0;
 }
 

@@ -364,6 +364,27 @@ def test_attention_over_cache_and_new_rows(shape, dtype, kind):
 
 
 @pytest.mark.parametrize("shape", [
+    # past, new, heads, kv heads, head_dim, page, window: the blocks a query tile's keys are shared out to
+    dict(past=[700, 0, 3000], new=[41, 5, 70], n_heads=8, n_kv_heads=4, head_dim=256, page_size=64, window=None),     # 8, one sequence with a single key tile
+    dict(past=[1000, 20], new=[30, 200], n_heads=5, n_kv_heads=1, head_dim=64, page_size=128, window=300),           # 8, two tiles a page, a window
+    dict(past=[333], new=[500], n_heads=6, n_kv_heads=3, head_dim=80, page_size=48, window=None),                    # 4, pages that tiles straddle
+    dict(past=[64], new=[1200], n_heads=6, n_kv_heads=2, head_dim=128, page_size=64, window=None),                   # 2
+    dict(past=[100], new=[1300], n_heads=8, n_kv_heads=8, head_dim=32, page_size=64, window=200),                    # none
+])
+def test_prefill_attention_shares_the_keys_among_blocks(shape):
+    c = Case(dtype=torch.bfloat16, seed=34, **shape)
+    b = c.batch("past")
+    sinks = rnd((c.n_heads,), torch.float32, 35)
+    for extra in ({}, {"sinks": sinks}, {"sigmoid_bias": sinks - 5.0}):
+        got = ops.attention(c.qkv, b, c.pages, new_kv=c.new_kv(), kind="prefill", **c.kw(softcap=5.0), **extra)
+        want = ops.attention(c.qkv, b, c.pages, new_kv=c.new_kv(), kind="plain", **c.kw(softcap=5.0), **extra)
+        assert_close(got, want, torch.bfloat16, rel=6.0, what=f"{list(extra)} against the plain kernel")
+    got = ops.attention(c.qkv, b, c.pages, new_kv=c.new_kv(), kind="prefill", **c.kw(softcap=5.0))
+    want = ref.attention_vectorised(c.qkv, b, c.pages, new_kv=c.new_kv(), **c.kw(softcap=5.0))
+    assert_close(got, want, torch.bfloat16, rel=6.0, what="against float64")
+
+
+@pytest.mark.parametrize("shape", [
     dict(past=[700, 0, 31], new=[1, 300, 2], n_heads=4, n_kv_heads=2, head_dim=512, page_size=64, window=None),   # several blocks of keys a warp
     dict(past=[520, 255], new=[3, 1], n_heads=3, n_kv_heads=1, head_dim=36, page_size=16, window=270),            # a first block cut by the window
     dict(past=[40], new=[2], n_heads=2, n_kv_heads=2, head_dim=10, page_size=16, window=None),                    # rows that are not 16-byte chunks
