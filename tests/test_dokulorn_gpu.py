@@ -258,6 +258,17 @@ def test_decay_attention_token_by_token(dtype, case):
     assert torch.equal(st2, st)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("case", [
+    dict(H=2, dim=100, vdim=132, lens=[3, 1], past=[0, 4], rot_n=100, silu=True, k_scale=0.1, decays=[0.9, 0.99]),
+    dict(H=1, dim=128, vdim=64, lens=[1, 1, 1, 1, 1], past=[0, 9, 3, 0, 70], rot_n=0, silu=False, k_scale=0.1, decays=[0.98]),
+    dict(H=2, dim=5, vdim=4, lens=[1, 1], past=[2, 0], rot_n=4, silu=False, k_scale=0.5, decays=[0.5, 0.7]),
+])
+def test_decay_attention_in_steps_of_single_tokens(dtype, case):
+    """The kernel of single-token steps: every number of rows a thread holds, columns that end inside a block's 64."""
+    test_decay_attention_token_by_token(dtype, case)
+
+
 @pytest.mark.parametrize("case", [
     dict(H=2, dim=64, vdim=64, lens=[64], past=[0], rot_n=64, silu=False, k_scale=0.125, decays=[0.98, 0.999]),
     dict(H=2, dim=32, vdim=96, lens=[200, 1, 65, 63], past=[0, 9, 0, 130], rot_n=16, silu=True, k_scale=1.0, decays=[0.6, 1.0]),
