@@ -373,6 +373,120 @@ __global__ void __launch_bounds__(PAIR_WARPS * 32) moe_down_combine_kernel(T* __
     if (lane == 0) out[(long long)t * width + n] = from_float<T>(total);
 }
 
+// ---- few pairs: an expert's matrices read once for all rows that chose it ----
+//
+// A step of a few tokens often has an expert chosen by several of them (8 rows x 6 of 64: 48 pairs, 35 experts), and the
+// kernel above reads its matrices once a pair: 403 MB instead of 293 through L2, which is what bounds it (62 us, 6.5 TB/s).
+// Here the first pair of an expert takes all its rows with it.  A warp asks for its weights (16-byte pieces, raw) before
+// it looks at the rows.  Every sum runs over the same values in the same order as above, so the results are the same bits.
+// 48 pairs of 64 gated experts of 1,024 x 2,048: 62 -> 53.5 us (eight pieces of each row in flight, two blocks a
+// multiprocessor: 65.6).  Experts of two matrices stay above: 16 pairs of 32 took 16.6 us here and 13.3 there.  So does the
+// down product: a block that took all rows' pairs for four outputs took 54 us and not 32.
+constexpr int SHARED_PAIRS = 128;          // most pairs of the step: four ballots find an expert's
+constexpr int SHARED_ROWS = 4;             // rows a warp sums at a time (with more the weights come again, from L2)
+constexpr int SHARED_PIECES = 4;           // 16-byte pieces of each of the two weight rows a lane has in flight
+
+template <typename T> __device__ __forceinline__ void unpack(const uint4& raw, float (&f)[Piece<T>::N]);
+template <> __device__ __forceinline__ void unpack<__nv_bfloat16>(const uint4& raw, float (&f)[8]) {
+    f[0] = __uint_as_float(raw.x << 16); f[1] = __uint_as_float(raw.x & 0xffff0000u);
+    f[2] = __uint_as_float(raw.y << 16); f[3] = __uint_as_float(raw.y & 0xffff0000u);
+    f[4] = __uint_as_float(raw.z << 16); f[5] = __uint_as_float(raw.z & 0xffff0000u);
+    f[6] = __uint_as_float(raw.w << 16); f[7] = __uint_as_float(raw.w & 0xffff0000u);
+}
+template <> __device__ __forceinline__ void unpack<float>(const uint4& raw, float (&f)[4]) {
+    f[0] = __uint_as_float(raw.x); f[1] = __uint_as_float(raw.y); f[2] = __uint_as_float(raw.z); f[3] = __uint_as_float(raw.w);
+}
+
+// The pairs of an expert as a set of bits, and taking the lowest one out of it (-1: empty).  Uniform over the warp.
+struct PairSet {
+    uint32_t bits[SHARED_PAIRS / 32];
+    __device__ __forceinline__ int take() {
+#pragma unroll
+        for (int i = 0; i < SHARED_PAIRS / 32; ++i)
+            if (bits[i]) {
+                const int b = __ffs(bits[i]) - 1;
+                bits[i] &= bits[i] - 1;
+                return 32 * i + b;
+            }
+        return -1;
+    }
+};
+template <typename T>
+__global__ void __launch_bounds__(PAIR_WARPS * 32) moe_gate_up_shared_kernel(T* __restrict__ mid, const T* __restrict__ x, const T* __restrict__ w,
+                                                                             const int* __restrict__ sel, const float* __restrict__ sel_w, int top,
+                                                                             int n_pairs, int n_real, int ff, int width, int activation, float act_param) {
+    constexpr int N = Piece<T>::N, SPAN = SHARED_PIECES * 32 * N;
+    rdl_grid_wait();
+    rdl_grid_launch_dependents();
+    const int lane = threadIdx.x & 31, j = blockIdx.x * PAIR_WARPS + (threadIdx.x >> 5);
+    const int p0 = blockIdx.y;
+    // all pairs' experts in one trip: this block's own among them
+    int mine[SHARED_PAIRS / 32], e = -1;
+    PairSet set;
+#pragma unroll
+    for (int i = 0; i < SHARED_PAIRS / 32; ++i) mine[i] = lane + 32 * i < n_pairs ? sel[lane + 32 * i] : -1;
+#pragma unroll
+    for (int i = 0; i < SHARED_PAIRS / 32; ++i) {
+        const int v = __shfl_sync(0xffffffffu, mine[i], p0 & 31);
+        if (i == p0 >> 5) e = v;
+    }
+#pragma unroll
+    for (int i = 0; i < SHARED_PAIRS / 32; ++i) set.bits[i] = __ballot_sync(0xffffffffu, mine[i] == e);
+    if (e < 0 || e >= n_real || j >= ff) return;
+    if (set.take() != p0) return;                          // an earlier pair has this expert's rows
+    const T* wg = w + ((long long)e * 2 * ff + j) * width;
+    const T* wu = wg + (long long)ff * width;
+    int next = p0;
+    while (next >= 0) {
+        int pair[SHARED_ROWS];
+#pragma unroll
+        for (int r = 0; r < SHARED_ROWS; ++r) { pair[r] = next; if (next >= 0) next = set.take(); }
+        float g[SHARED_ROWS], u[SHARED_ROWS];
+#pragma unroll
+        for (int r = 0; r < SHARED_ROWS; ++r) g[r] = u[r] = 0.f;
+        for (int i0 = lane * N; i0 < width; i0 += SPAN) {
+            uint4 rg[SHARED_PIECES], ru[SHARED_PIECES];
+#pragma unroll
+            for (int i = 0; i < SHARED_PIECES; ++i) {
+                rg[i] = ru[i] = make_uint4(0u, 0u, 0u, 0u);
+                if (i0 + i * 32 * N < width) {
+                    rg[i] = __ldg(reinterpret_cast<const uint4*>(wg + i0 + i * 32 * N));
+                    ru[i] = __ldg(reinterpret_cast<const uint4*>(wu + i0 + i * 32 * N));
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < SHARED_ROWS; ++r) {
+                if (pair[r] < 0) break;
+                const T* row = x + (long long)(pair[r] / top) * width;
+#pragma unroll
+                for (int i = 0; i < SHARED_PIECES; ++i) {
+                    if (i0 + i * 32 * N >= width) break;
+                    float xv[N], a[N], b[N];
+                    Piece<T>::load(row + i0 + i * 32 * N, xv);
+                    unpack<T>(rg[i], a);
+                    unpack<T>(ru[i], b);
+#pragma unroll
+                    for (int k = 0; k < N; ++k) { g[r] = fmaf(a[k], xv[k], g[r]); u[r] = fmaf(b[k], xv[k], u[r]); }
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < SHARED_ROWS; ++r) {
+            if (pair[r] < 0) break;
+            const float in_w = sel_w ? sel_w[pair[r]] : 1.0f;
+            const float y = rdl_gated(warp_sum(g[r]) * in_w, warp_sum(u[r]) * in_w, activation, act_param);
+            if (lane == 0) mid[(long long)pair[r] * ff + j] = from_float<T>(y);
+        }
+    }
+}
+
+// Whether a step's pairs take the shared form: few enough, rows in whole 16-byte pieces, and enough of them that experts
+// repeat.  Taking the rows together costs registers and with them loads in flight, about an eighth of the time, so it
+// pays from about as many repeated pairs on; with half as many pairs as experts a fifth repeats.
+static bool shared_ok(int dtype, long long n_pairs, int n_real, int n, const void* a, const void* b) {
+    return n_pairs <= SHARED_PAIRS && 2 * n_pairs >= n_real && n % (dtype == RDL_BF16 ? 8 : 4) == 0 && (((uintptr_t)a | (uintptr_t)b) & 15) == 0;
+}
+
 // ---- many rows: sorted by expert, one expert per tile of MOE_TILE rows ----
 
 constexpr int MOE_TILE = 128, ALIGN_THREADS = 1024;
@@ -541,6 +655,15 @@ extern "C" int rdl_moe_gate_up(void* mid, int dtype, const void* x, const void* 
     RDL_REQUIRE((long long)n_rows * top <= 65535, "moe_gate_up: %d rows x %d choices exceed the grid limit", n_rows, top);
     const dim3 grid((ff + PAIR_WARPS - 1) / PAIR_WARPS, n_rows * top);
     cudaStream_t st = (cudaStream_t)stream;
+    if (activation < 16 && shared_ok(dtype, (long long)n_rows * top, n_real, width, x, w_gate_up)) {
+        if (dtype == RDL_BF16)
+            RDL_CHECK_EX(rdl_launch(moe_gate_up_shared_kernel<__nv_bfloat16>, grid, dim3(PAIR_WARPS * 32), 0, st, (__nv_bfloat16*)mid, (const __nv_bfloat16*)x,
+                                    (const __nv_bfloat16*)w_gate_up, sel, sel_w, top, n_rows * top, n_real, ff, width, activation, act_param), "moe_gate_up");
+        else
+            RDL_CHECK_EX(rdl_launch(moe_gate_up_shared_kernel<float>, grid, dim3(PAIR_WARPS * 32), 0, st, (float*)mid, (const float*)x, (const float*)w_gate_up,
+                                    sel, sel_w, top, n_rows * top, n_real, ff, width, activation, act_param), "moe_gate_up");
+        return 0;
+    }
     if (dtype == RDL_BF16)
         RDL_CHECK_EX(rdl_launch(moe_gate_up_kernel<__nv_bfloat16>, grid, dim3(PAIR_WARPS * 32), 0, st, (__nv_bfloat16*)mid, (const __nv_bfloat16*)x,
                                 (const __nv_bfloat16*)w_gate_up, sel, sel_w, top, n_real, ff, width, activation, act_param), "moe_gate_up");

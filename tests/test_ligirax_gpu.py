@@ -389,3 +389,22 @@ def test_command_line_generates_with_a_ligirax_folder(capsys):
     assert "arch=Ligirax" in capsys.readouterr().err
     gen = Generator(lh.loaded_model(name, "float32"), max_batch=1, max_context=64).with_temperature(0.0)
     assert [int(t) for t in out.getvalue().split()] == gen.generate(p, 6)[len(p):]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,top,n_real,identity,ff,width", [(16, 3, 40, 2, 24, 1160), (11, 4, 33, 0, 9, 8), (16, 8, 60, 5, 5, 4104), (7, 3, 40, 0, 16, 48)])
+def test_experts_whose_rows_are_taken_together(dtype, rows, top, n_real, identity, ff, width):
+    """Steps in which experts repeat (one of them in every row: more rows than a warp sums at a time) give the bits of the
+    same rows one at a time, where every pair streams its expert's matrices itself."""
+    from rust_deeplearning_b200.kernels import ops
+    g = torch.Generator().manual_seed(5)
+    sel = torch.stack([torch.cat([torch.tensor([n_real // 2]), 1 + n_real // 2 + torch.randperm(n_real + identity - 1 - n_real // 2, generator=g)[:top - 1]])
+                       for _ in range(rows)]).to(torch.int32).to(DEV)
+    assert rows * top <= 128 and (2 * rows * top >= n_real) and 2 * top < n_real
+    rnd = lambda *s: (torch.randn(s, generator=g) * 0.3).to(dtype).to(DEV)
+    x, gu, dn, sel_w = rnd(rows, width), rnd(n_real, 2 * ff, width), rnd(n_real, width, ff), torch.rand((rows, top), generator=g).to(DEV)
+    for on_input in (False, True):
+        got = ops.moe_experts_few(x, sel, sel_w, gu, dn, n_real, "silu", 0.0, weights_on_input=on_input)
+        one = [ops.moe_experts_few(x[t:t + 1], sel[t:t + 1].contiguous(), sel_w[t:t + 1].contiguous(), gu, dn, n_real, "silu", 0.0, weights_on_input=on_input)
+               for t in range(rows)]
+        assert torch.equal(got, torch.cat(one))
