@@ -208,6 +208,94 @@ __global__ void __launch_bounds__(128) short_conv_kernel(const T* __restrict__ i
     }
 }
 
+// Four taps over many rows (a prompt): a thread takes 16 bytes of channels and four rows, whose seven inputs it loads once; the
+// kernel above loads two bytes at a time and every input four times.  Every output goes through the same operations.
+// Four prompts of 3,400 rows with two such layers and 16 single-token steps: 9.70 -> 9.51 ms.
+constexpr int CONV_RUN = 4;
+template <typename T>
+__global__ void __launch_bounds__(128) short_conv4_rows_kernel(const T* __restrict__ in, long long in_stride, int n_rows, int channels,
+                                                               const T* __restrict__ w, const void* __restrict__ b, int b_dtype, int silu,
+                                                               float* __restrict__ state, const int* __restrict__ tok_seq,
+                                                               const int* __restrict__ tok_pos, const int* __restrict__ seq_start,
+                                                               const int* __restrict__ slots, T* __restrict__ out) {
+    constexpr int N = 16 / (int)sizeof(T), TAPS = 4, KEEP = TAPS - 1;
+    rdl_grid_wait();
+    rdl_grid_launch_dependents();
+    const int t0 = blockIdx.x * CONV_RUN, c0 = (blockIdx.y * blockDim.x + threadIdx.x) * N;
+    if (c0 >= channels) return;
+    auto load = [&](const T* p, float (&f)[N]) {
+#pragma unroll
+        for (int i = 0; i < N; i += 4) {
+            float g[4];
+            rn_load4(p + i, g);
+            f[i] = g[0]; f[i + 1] = g[1]; f[i + 2] = g[2]; f[i + 3] = g[3];
+        }
+    };
+    auto store = [&](int t, const float (&f)[N]) {
+#pragma unroll
+        for (int i = 0; i < N; i += 4) {
+            const float g[4] = {f[i], f[i + 1], f[i + 2], f[i + 3]};
+            rn_store4(out + (long long)t * channels + c0 + i, g);
+        }
+    };
+    float x[CONV_RUN + KEEP][N], wt[TAPS][N], bias[N];
+#pragma unroll
+    for (int i = 0; i < CONV_RUN + KEEP; ++i) {            // rows t0 - 3 .. t0 + 3; which of them are a row's own inputs shows below
+        const int t = t0 + i - KEEP;
+        if (t >= 0 && t < n_rows) load(in + (long long)t * in_stride + c0, x[i]);
+    }
+#pragma unroll
+    for (int j = 0; j < TAPS; ++j) {                       // the weights lie channel by channel
+        float f[N];
+        load(w + (long long)c0 * TAPS + j * N, f);
+#pragma unroll
+        for (int i = 0; i < N; ++i) wt[(j * N + i) % TAPS][(j * N + i) / TAPS] = f[i];
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) bias[i] = b ? rdl_load(b, c0 + i, b_dtype) : 0.f;
+#pragma unroll
+    for (int u = 0; u < CONV_RUN; ++u) {
+        const int t = t0 + u;
+        if (t >= n_rows) break;
+        const int p = tok_pos[t];
+        float acc[N];
+#pragma unroll
+        for (int i = 0; i < N; ++i) acc[i] = p < 0 ? 0.f : bias[i];
+        if (p < 0) { store(t, acc); continue; }
+        const int seq = tok_seq[t], row0 = seq_start[seq], r = t - row0;
+        if (r >= KEEP) {
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j)
+#pragma unroll
+                for (int i = 0; i < N; ++i) acc[i] = fmaf(wt[j][i], x[u + j][i], acc[i]);
+            if (silu) {
+#pragma unroll
+                for (int i = 0; i < N; ++i) acc[i] = silu_exact(acc[i]);
+            }
+            store(t, acc);
+        } else if (r == 0) {
+            // a sequence's first rows, which read the slot, and the slot's new rows: channel by channel as above
+            const int n = seq_start[seq + 1] - row0;
+            float* st = state + (long long)slots[seq] * KEEP * channels;
+            for (int i = 0; i < N; ++i) {
+                const int c = c0 + i;
+                float old[CONV_MAX_TAPS], wc[CONV_MAX_TAPS];
+                for (int j = 0; j < TAPS; ++j) wc[j] = to_float(w[(long long)c * TAPS + j]);
+                for (int j = 0; j < KEEP; ++j) old[j] = p > 0 ? st[(long long)j * channels + c] : 0.f;
+                const float bc = b ? rdl_load(b, c, b_dtype) : 0.f;
+                for (int rr = 0; rr < min(n, KEEP); ++rr) conv_row<T>(in, in_stride, row0, rr, p, c, channels, TAPS, wc, bc, silu, old, out);
+                for (int j = 0; j < KEEP; ++j) {
+                    const int src = n - KEEP + j;
+                    float v;
+                    if (src >= 0) v = to_float(in[(long long)(row0 + src) * in_stride + c]);
+                    else v = p + src < 0 ? 0.f : old[KEEP + src];
+                    st[(long long)j * channels + c] = v;
+                }
+            }
+        }
+    }
+}
+
 template <typename T>
 __global__ void gated_residual_kernel(float* __restrict__ res, const T* __restrict__ gates, long long gates_stride,
                                       const void* __restrict__ bias_a, const void* __restrict__ bias_b, int bias_dtype,
@@ -338,6 +426,18 @@ extern "C" int rdl_short_conv(const void* in, long long in_stride, int dtype, in
     RDL_REQUIRE((channels + 127) / 128 <= 65535, "short_conv: too many channels for one grid");
     const dim3 grid(n_rows, (channels + 127) / 128), block(128);
     cudaStream_t st = (cudaStream_t)stream;
+    const int piece = dtype == RDL_BF16 ? 8 : 4;
+    // (few rows: there the form above, a thread a channel, has more threads for the rows that read the slot)
+    if (n_rows >= 512 && taps == 4 && w_dtype == dtype && channels % piece == 0 && in_stride % piece == 0 && aligned16(in) && aligned16(w) && aligned16(out)) {
+        const dim3 runs((n_rows + CONV_RUN - 1) / CONV_RUN, (channels / piece + 127) / 128);
+        if (dtype == RDL_BF16)
+            RDL_CHECK_EX(rdl_launch(short_conv4_rows_kernel<__nv_bfloat16>, runs, block, 0, st, (const __nv_bfloat16*)in, in_stride, n_rows, channels,
+                                    (const __nv_bfloat16*)w, bias, w_dtype, silu, state, tok_seq, tok_pos, seq_start, slots, (__nv_bfloat16*)out), "short_conv");
+        else
+            RDL_CHECK_EX(rdl_launch(short_conv4_rows_kernel<float>, runs, block, 0, st, (const float*)in, in_stride, n_rows, channels, (const float*)w, bias,
+                                    w_dtype, silu, state, tok_seq, tok_pos, seq_start, slots, (float*)out), "short_conv");
+        return 0;
+    }
     if (dtype == RDL_BF16)
         RDL_CHECK_EX(rdl_launch(short_conv_kernel<__nv_bfloat16>, grid, block, 0, st, (const __nv_bfloat16*)in, in_stride, channels, taps, w, w_dtype,
                                 bias, silu, state, tok_seq, tok_pos, seq_start, slots, (__nv_bfloat16*)out), "short_conv");

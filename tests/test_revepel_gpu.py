@@ -100,6 +100,13 @@ def test_norm_and_token_shift_at_every_depth(dtype, width):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("channels,lens,past,bias", [(40, [1, 2, 3, 300, 1, 4, 205, 6], [0, 1, 2, 0, 9, 0, 4, 0], True), (1048, [513], [0], False), (8, [700, 5], [3, 1], True)])
+def test_short_convolution_of_many_rows(dtype, channels, lens, past, bias):
+    """Four taps over more rows than 512: runs of four rows that sequences of every length begin and end in."""
+    test_short_convolution_with_carried_inputs(dtype, 4, channels, lens, past, bias)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("taps,channels,lens,past,bias", [(4, 40, [9, 1, 2, 1], [0, 5, 0, 0], True), (2, 130, [3, 30], [1, 0], False),
                                                           (1, 24, [4], [2], True), (3, 300, [1, 2, 70], [1, 1, 2], False), (8, 16, [3, 20], [0, 4], True)])
 def test_short_convolution_with_carried_inputs(dtype, taps, channels, lens, past, bias):
