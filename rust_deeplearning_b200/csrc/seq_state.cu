@@ -69,35 +69,47 @@ __global__ void __launch_bounds__(256) norm_shift_kernel(const float* __restrict
     }
 }
 
-// The same with a row in registers (NIT groups of four values a thread).  The kernel is bound by latency: a row's sum,
-// the sum of the one other row its block may need (the row before it, or for a sequence's first row the sequence's
-// last) and the element-wise pass each went to memory in turn, element after element.  Here the constants are
-// asked for before the wait, the rows, the batch description and the slot's state in three trips, and both sums meet
-// in one exchange.  Every row is summed in the same order whichever block does it, so cuts stay invisible.
-// Width 2048, 4 rows of a single-token step: 23.6 -> 7.8 us a launch, the wait for the kernel before included.
+// A thread's values of a row, all asked for before one is used: no branch and no conversion between the loads (a place beyond
+// the row reads its last value, which nothing uses).
+template <int NIT, typename S>
+__device__ __forceinline__ void row_load(const S* __restrict__ p, int width, float (&f)[NIT]) {
+    S raw[NIT];
+#pragma unroll
+    for (int it = 0; it < NIT; ++it) raw[it] = p[min((int)(threadIdx.x + it * blockDim.x), width - 1)];
+#pragma unroll
+    for (int it = 0; it < NIT; ++it) f[it] = to_float(raw[it]);
+}
+template <int NIT>
+__device__ __forceinline__ void row_load(const void* p, int dtype, int width, float (&f)[NIT]) {
+    if (dtype == RDL_BF16) row_load<NIT>((const __nv_bfloat16*)p, width, f);
+    else row_load<NIT>((const float*)p, width, f);
+}
+
+// The same with a row in registers: thread i holds values i, i + threads, ... (NIT of them at most).  The kernel is bound by
+// latency: a row's sum, the sum of the one other row its block may need (the row before it, or for a sequence's first row
+// the sequence's last) and the element-wise pass each went to memory in turn, element after element.  Here the
+// constants are asked for before the wait, the rows, the batch description and the slot's state in three trips, and both
+// sums meet in one exchange.  Every sum takes the order of the kernel above (a thread's values from the first on, the warp's
+// lanes, the warps as the lanes of one), so both give the same bits, whichever block does it.  Groups of four values a
+// thread load wider and sum in another order; they are no faster where it counts.
+// Width 2,048, bfloat16: 3,399 rows 30.7 us in the kernel above, 22.5 in groups of four, 21.5 here; four prompts of 200 to
+// 1,500 rows and 16 single-token steps of a model of four such layers 10.76, 9.45 and 9.49 ms.
 template <typename T, int NIT>
-__global__ void __launch_bounds__(256) norm_shift_vec_kernel(const float* __restrict__ x, const void* __restrict__ w, int w_dtype, float eps,
+__global__ void __launch_bounds__(256) norm_shift_row_kernel(const float* __restrict__ x, const void* __restrict__ w, int w_dtype, float eps,
                                                              const void* __restrict__ shift, int shift_dtype, float* __restrict__ state,
                                                              const int* __restrict__ tok_seq, const int* __restrict__ tok_pos,
                                                              const int* __restrict__ seq_start, const int* __restrict__ slots,
                                                              T* __restrict__ normed, T* __restrict__ mixed, int width) {
     __shared__ float2 sums[8];
     const int t = blockIdx.x, tid = threadIdx.x, n_thr = blockDim.x;
-    float wv[NIT][4], sh[NIT][4], own[NIT][4], other[NIT][4], old[NIT][4];
-#pragma unroll
-    for (int it = 0; it < NIT; ++it) {
-        const int e = (tid + it * n_thr) * 4;
-        if (e < width) { rn_load4(w, e, w_dtype, wv[it]); rn_load4(shift, e, shift_dtype, sh[it]); }
-    }
+    float wv[NIT], sh[NIT], own[NIT], other[NIT], old[NIT];
+    row_load<NIT>(w, w_dtype, width, wv);
+    row_load<NIT>(shift, shift_dtype, width, sh);
     rdl_grid_wait();
     rdl_grid_launch_dependents();
     const int p = tok_pos[t], seq = tok_seq[t];
     const float* xr = x + (long long)t * width;
-#pragma unroll
-    for (int it = 0; it < NIT; ++it) {
-        const int e = (tid + it * n_thr) * 4;
-        if (e < width) rn_load4(xr + e, own[it]);
-    }
+    row_load<NIT>(xr, width, own);
     bool first = false, more = false;      // the sequence's first row of the step; it has further rows
     float* st = nullptr;
     if (p >= 0) {                          // (a padding row of a fixed-size batch has finite values and no slot)
@@ -106,51 +118,36 @@ __global__ void __launch_bounds__(256) norm_shift_vec_kernel(const float* __rest
         first = t == row0;
         more = first && row_end - 1 != t;
         const float* xo = first ? x + (long long)(row_end - 1) * width : xr - width;
-#pragma unroll
-        for (int it = 0; it < NIT; ++it) {
-            const int e = (tid + it * n_thr) * 4;
-            if (e < width) {
-                if (!first || more) rn_load4(xo + e, other[it]);
-                if (first && p > 0) rn_load4(st + e, old[it]);
-            }
-        }
+        if (!first || more) row_load<NIT>(xo, width, other);
+        if (first && p > 0) row_load<NIT>(st, width, old);
     }
     const bool has_other = p >= 0 && (!first || more);
     float s0 = 0.f, s1 = 0.f;
 #pragma unroll
     for (int it = 0; it < NIT; ++it) {
-        const int e = (tid + it * n_thr) * 4;
-        if (e < width) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                s0 = fmaf(own[it][k], own[it][k], s0);
-                if (has_other) s1 = fmaf(other[it][k], other[it][k], s1);
-            }
+        if (tid + it * n_thr < width) {
+            s0 = fmaf(own[it], own[it], s0);
+            if (has_other) s1 = fmaf(other[it], other[it], s1);
         }
     }
     s0 = warp_sum(s0);
     s1 = warp_sum(s1);
     if ((tid & 31) == 0) sums[tid >> 5] = make_float2(s0, s1);
     __syncthreads();
-    s0 = s1 = 0.f;
-    for (int i = 0; i < n_thr >> 5; ++i) { s0 += sums[i].x; s1 += sums[i].y; }
+    const bool a_warps = (tid & 31) < n_thr >> 5;
+    s0 = warp_sum(a_warps ? sums[tid & 31].x : 0.f);
+    s1 = warp_sum(a_warps ? sums[tid & 31].y : 0.f);
     const float inv = 1.0f / sqrtf(s0 / (float)width + eps), inv_other = 1.0f / sqrtf(s1 / (float)width + eps);
 #pragma unroll
     for (int it = 0; it < NIT; ++it) {
-        const int e = (tid + it * n_thr) * 4;
+        const int e = tid + it * n_thr;
         if (e >= width) continue;
-        float n[4], m[4], keep[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            n[k] = own[it][k] * inv * wv[it][k];
-            const float o = has_other ? other[it][k] * inv_other * wv[it][k] : n[k];     // the row before, or the sequence's last
-            const float prev = first ? (p == 0 ? 0.f : old[it][k]) : o;
-            m[k] = p < 0 ? n[k] : n[k] + (prev - n[k]) * sh[it][k];
-            keep[k] = o;
-        }
-        rn_store4(normed + (long long)t * width + e, n);
-        rn_store4(mixed + (long long)t * width + e, m);
-        if (first) rn_store4(st + e, keep);
+        const float n = own[it] * inv * wv[it];
+        const float o = has_other ? other[it] * inv_other * wv[it] : n;      // the row before, or the sequence's last
+        const float prev = first ? (p == 0 ? 0.f : old[it]) : o;
+        normed[(long long)t * width + e] = from_float<T>(n);
+        mixed[(long long)t * width + e] = from_float<T>(p < 0 ? n : n + (prev - n) * sh[it]);
+        if (first) st[e] = o;
     }
 }
 
@@ -387,24 +384,20 @@ extern "C" int rdl_norm_shift(const float* x, const void* w, int w_dtype, float 
                 "norm_shift: bad arguments");
     if (n_rows == 0) return 0;
     cudaStream_t st = (cudaStream_t)stream;
-    const int vt = vec_threads(width);
-    if (vec_ok(width, vt) && aligned16(x) && aligned16(w) && aligned16(shift) && aligned16(state) && aligned16(normed) && aligned16(mixed)) {
+    const dim3 grid(n_rows), block(width <= 512 ? 64 : (width <= 2048 ? 128 : 256));
+    if (width <= 8192) {                     // a thread's share of a row fits its registers
         cudaError_t e;
-#define NORM_SHIFT_LAUNCH(N)                                                                                                           \
-    do {                                                                                                                               \
-        if (out_dtype == RDL_BF16)                                                                                                     \
-            e = rdl_launch(norm_shift_vec_kernel<__nv_bfloat16, N>, dim3(n_rows), dim3(vt), 0, st, x, w, w_dtype, eps, shift,          \
-                           shift_dtype, state, tok_seq, tok_pos, seq_start, slots, (__nv_bfloat16*)normed, (__nv_bfloat16*)mixed, width); \
-        else                                                                                                                           \
-            e = rdl_launch(norm_shift_vec_kernel<float, N>, dim3(n_rows), dim3(vt), 0, st, x, w, w_dtype, eps, shift, shift_dtype,     \
-                           state, tok_seq, tok_pos, seq_start, slots, (float*)normed, (float*)mixed, width);                           \
-    } while (0)
-        RN_BY_DEPTH(vec_depth(width, vt), NORM_SHIFT_LAUNCH)
+#define NORM_SHIFT_LAUNCH(T, N)                                                                                                          \
+    rdl_launch(norm_shift_row_kernel<T, N>, grid, block, 0, st, x, w, w_dtype, eps, shift, shift_dtype, state, tok_seq, tok_pos, seq_start, \
+               slots, (T*)normed, (T*)mixed, width)
+#define NORM_SHIFT_BY_DEPTH(T) (width <= 512 ? NORM_SHIFT_LAUNCH(T, 8) : width <= 4096 ? NORM_SHIFT_LAUNCH(T, 16) : NORM_SHIFT_LAUNCH(T, 32))
+        if (out_dtype == RDL_BF16) e = NORM_SHIFT_BY_DEPTH(__nv_bfloat16);
+        else e = NORM_SHIFT_BY_DEPTH(float);
+#undef NORM_SHIFT_BY_DEPTH
 #undef NORM_SHIFT_LAUNCH
         RDL_CHECK_EX(e, "norm_shift");
         return 0;
     }
-    const dim3 grid(n_rows), block(width <= 512 ? 64 : (width <= 2048 ? 128 : 256));
     if (out_dtype == RDL_BF16)
         RDL_CHECK_EX(rdl_launch(norm_shift_kernel<__nv_bfloat16>, grid, block, 0, st, x, w, w_dtype, eps, shift, shift_dtype, state, tok_seq, tok_pos,
                                 seq_start, slots, (__nv_bfloat16*)normed, (__nv_bfloat16*)mixed, width), "norm_shift");

@@ -94,9 +94,36 @@ def test_norm_and_token_shift(dtype, width, lens, past):
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("width", [4, 30, 260, 2048, 8192, 8196])
 def test_norm_and_token_shift_at_every_depth(dtype, width):
-    """Rows held in registers at each depth (one group of four values a thread up to eight), and the widths beside them
-    that are no multiple of four or too wide."""
+    """Rows held in registers at each depth, the widest, and the width beside it."""
     test_norm_and_token_shift(dtype, width, [1, 3, 1, 2], [6, 0, 0, 2])
+
+
+@pytest.mark.parametrize("width", [4, 30, 300, 512, 520, 2048, 2052, 4608, 8192, 8196])
+def test_norm_and_token_shift_sums_a_row_in_one_order(width):
+    """A row's sum of squares is taken by `threads` (64, 128, 256 by the width) in steps of `threads`, then over the lanes, then
+    over the warps, whatever the row's place in its sequence: the normed rows are those bits.  (The fused multiply-add is
+    formed in 64 bits, where the product is exact.)"""
+    threads = 64 if width <= 512 else 128 if width <= 2048 else 256
+    r = Rows([1, 3, 2], [6, 0, 2])
+    x, w = rnd((r.T, width), torch.float32, 1, 3.0), rnd((width,), torch.float32, 2, 0.3) + 1.0
+    xn = x.cpu().numpy()
+    padded = np.zeros((r.T, -(-width // threads) * threads), dtype=np.float32)
+    padded[:, :width] = xn
+    acc = np.zeros((r.T, threads), dtype=np.float32)
+    for part in np.split(padded, padded.shape[1] // threads, axis=1):
+        acc = (part.astype(np.float64) * part + acc).astype(np.float32)
+
+    def lanes(v):                            # [..., 32] -> [...]: halves of the warp added pair by pair
+        for o in (16, 8, 4, 2, 1):
+            v = v[..., :o] + v[..., o:2 * o]
+        return v[..., 0]
+
+    warps = np.zeros((r.T, 32), dtype=np.float32)
+    warps[:, :threads // 32] = lanes(acc.reshape(r.T, threads // 32, 32))
+    inv = np.float32(1) / np.sqrt(lanes(warps) / np.float32(width) + np.float32(1e-5))
+    state = torch.zeros((r.n_slots, width), dtype=torch.float32, device=DEV)
+    n, _ = ops.norm_shift(x, w, 1e-5, w, state, tok_seq=r.tok_seq, out_dtype=torch.float32, **r.where())
+    assert np.array_equal(n.cpu().numpy(), xn * inv[:, None] * w.cpu().numpy())
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
