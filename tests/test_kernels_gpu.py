@@ -397,6 +397,29 @@ def test_float32_attention_shares_the_keys_among_warps(shape):
     assert_close(got, want, torch.float32, what="float32 attention", f32_tol=c.max_total * 2.0 ** -24)     # sums over the keys
 
 
+@pytest.mark.parametrize("head_dim,n_heads,n_kv_heads,page_size,window,chunk", [
+    (256, 8, 4, 64, None, None), (256, 6, 3, 64, 300, None), (80, 8, 2, 48, None, None), (128, 8, 8, 128, None, 150), (64, 8, 1, 64, None, None),
+    (32, 8, 4, 16, 200, None), (16, 8, 4, 64, None, None)])
+def test_prefill_attention_has_the_same_bits_whatever_shares_the_step(head_dim, n_heads, n_kv_heads, page_size, window, chunk):
+    """All query tiles in one launch (more than fill the chip: a block each) against a few at a time, which clusters of 2, 4 and 8
+    blocks take: the order of a row's operations follows its position alone."""
+    c = Case(past=[700, 64, 0, 3000, 9], new=[41, 1500, 70, 100, 1], n_heads=n_heads, n_kv_heads=n_kv_heads, head_dim=head_dim, page_size=page_size,
+             window=window, dtype=torch.bfloat16, seed=36)
+    b = c.batch("past")
+    assert b.n_tiles * n_heads > 148
+    h = rnd((n_heads,), torch.float32, 35)
+    bias = ops.DistanceBias.of(rnd((n_heads, 100), torch.float32, 37))
+    rows = [slice(int(c.seq_start[s]) + int(q0), min(int(c.seq_start[s]) + int(q0) + 64, int(c.seq_start[s + 1])))
+            for s, q0 in zip(b.tile_seq.tolist(), b.tile_q0.tolist())]
+    for extra in ({}, {"sinks": h}, {"sigmoid_bias": h - 5.0}, {"distance_bias": bias}):
+        run = lambda at, n: ops.attention(c.qkv, b._replace(tile_seq=b.tile_seq[at:at + n], tile_q0=b.tile_q0[at:at + n], n_tiles=n), c.pages,
+                                          new_kv=c.new_kv(), kind="prefill", chunk=chunk, **c.kw(softcap=5.0), **extra)
+        whole = run(0, b.n_tiles)
+        for at, n in ((0, 1), (b.n_tiles - 3, 2), (b.n_tiles - 1, 1), (1, 5), (b.n_tiles - 8, 8), (2, 14)):
+            part = run(at, n)
+            assert all(torch.equal(part[r], whole[r]) for r in rows[at:at + n]), (list(extra), at, n)
+
+
 TC_SHAPES = [
     dict(new=[1], n_heads=1, n_kv_heads=1, head_dim=64, window=None),
     dict(new=[5, 129, 70], n_heads=4, n_kv_heads=2, head_dim=64, window=None),
