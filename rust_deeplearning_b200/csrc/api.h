@@ -11,7 +11,7 @@ extern "C" {
 #define RDL_ACT_SILU 1
 #define RDL_ACT_SWISH_LIMIT 2   // min(g, L) sigmoid(1.702 min(g, L)) (clamp(u, -L, L) + 1), L a parameter
 
-#define RDL_ABI_VERSION 21
+#define RDL_ABI_VERSION 22
 
 const char* rdl_last_error(void);
 int rdl_abi_version(void);
@@ -81,12 +81,16 @@ typedef struct {
     // decode kernel, optional: kv_share > 1 - so many consecutive of the n_kv_heads read the same key/value head of the cache
     // (a group of query heads too large for one block, cut into kv_share equal ones); not together with new_rows
     int kv_share;
+    // prefill kernel, optional: the most keys a query of the step sees (0: not known); how many blocks share a tile rests on it, results do not
+    int max_keys;
     // filled in by the launcher: clock cycles after which a wait is given up, and the test's extra bytes
     long long wait_cycles; int test_extra_tx;
 } AttentionArgs;
 
 int rdl_attention_plain(const AttentionArgs* a, void* stream);
 int rdl_attention_prefill(const AttentionArgs* a, void* stream);
+// how many blocks rdl_attention_prefill gives a query tile and head, of `pairs` of them in a launch on `sms` multiprocessors
+int rdl_attention_prefill_blocks(long long pairs, int head_dim, int sigmoid, int max_keys, int sms);
 int rdl_attention_decode(const AttentionArgs* a, void* stream);
 // prefill attention on tcgen05 tensor cores for sequences that start at position 0 and head sizes that are
 // multiples of 64; q, k_new and v_new must be the packed rows of one [tokens, row_width] buffer

@@ -17,6 +17,7 @@
 #include "launch.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace {
 
@@ -86,6 +87,9 @@ struct Tile {
     int pr0, pr1, lo0, lo1;                         // the thread's rows: position and first key
     int pw_first, pw_last, low_first, low_last;     // its warp's rows: the same, first and last
     const int* table;
+    int ksteps;
+    float inv_cap;
+    const float* rel;                               // distance bias of the head: entry n for distance n, the last one for all beyond
     __device__ __forceinline__ Tile(const AttentionArgs& a, int tile, int head) {
         h = head;
         seq = a.tile_seq[tile]; q0 = a.tile_q0[tile];
@@ -95,6 +99,9 @@ struct Tile {
         hd = a.head_dim;
         g = h / (a.n_heads / a.n_kv_heads);
         table = a.tables ? a.tables + (long long)seq * a.table_width : nullptr;
+        ksteps = (hd + 15) / 16;
+        inv_cap = a.softcap > 0.f ? 1.0f / a.softcap : 0.f;
+        rel = a.rel_bias ? a.rel_bias + (long long)h * a.rel_len : nullptr;
         const int warp = threadIdx.x >> 5, quad = (threadIdx.x & 31) >> 2;
         p_first = past + q0; p_last = past + q0 + rows - 1;
         lo_first = rdl_first_key(p_first, a.window, a.chunk);
@@ -161,9 +168,6 @@ template <int HD, int MODE, bool AHEAD>
 __device__ __forceinline__ void tile_scores(const AttentionArgs& a, const Tile& t, uint32_t sQ, uint32_t sK, int kv0, float (&s)[BN / 8][4],
                                             float& mx0, float& mx1) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tq = lane & 3;
-    const int ksteps = (t.hd + 15) / 16;
-    const float inv_cap = a.softcap > 0.f ? 1.0f / a.softcap : 0.f;
-    const float* rel = MODE == 2 ? a.rel_bias + (long long)t.h * a.rel_len : nullptr;      // entry n: distance n, the last one for all beyond
 #pragma unroll
     for (int i = 0; i < BN / 8; ++i) { s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.f; }
     if (AHEAD) {       // the next 16 values' operands are asked for before this one's products
@@ -182,16 +186,16 @@ __device__ __forceinline__ void tile_scores(const AttentionArgs& a, const Tile& 
             }
         };
         load(0, 0);
-        for (int kk = 0; kk < ksteps; kk += 2) {
-            if (kk + 1 < ksteps) load(1, kk + 1);
+        for (int kk = 0; kk < t.ksteps; kk += 2) {
+            if (kk + 1 < t.ksteps) load(1, kk + 1);
             multiply(0);
-            if (kk + 1 < ksteps) {
-                if (kk + 2 < ksteps) load(0, kk + 2);
+            if (kk + 1 < t.ksteps) {
+                if (kk + 2 < t.ksteps) load(0, kk + 2);
                 multiply(1);
             }
         }
     } else {
-        for (int kk = 0; kk < ksteps; ++kk) {
+        for (int kk = 0; kk < t.ksteps; ++kk) {
             uint32_t af[4];
             ldmatrix_x4(af, tile_addr<HD>(sQ, warp * 16 + (lane & 15), 2 * kk + (lane >> 4)));
 #pragma unroll
@@ -211,10 +215,10 @@ __device__ __forceinline__ void tile_scores(const AttentionArgs& a, const Tile& 
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             float v = s[nt][e] * a.score_scale;
-            if (a.softcap > 0.f) v = a.softcap * tanh_fast(v * inv_cap);
+            if (a.softcap > 0.f) v = a.softcap * tanh_fast(v * t.inv_cap);
             if (MODE == 2) {
                 const int dist = ((e < 2) ? t.pr0 : t.pr1) - (kv0 + nt * 8 + 2 * tq + (e & 1));
-                v = fmaf(v, LOG2E, __ldg(rel + (rel_plain ? dist : min(max(dist, 0), a.rel_len - 1))));
+                v = fmaf(v, LOG2E, __ldg(t.rel + (rel_plain ? dist : min(max(dist, 0), a.rel_len - 1))));
             } else {
                 v *= LOG2E;
             }
@@ -304,7 +308,7 @@ __device__ __forceinline__ void store_rows(const AttentionArgs& a, const Tile& t
 
 // MODE 0: softmax; 1: sigmoid weights; 2: softmax with a bias per head and distance (base-2 domain) added to the scores
 template <int HD, int MODE>
-__global__ void __launch_bounds__(NTHREADS) attention_prefill_kernel(AttentionArgs a) {
+__global__ void __launch_bounds__(NTHREADS, HD == 64 && MODE == 1 ? 4 : 0) attention_prefill_kernel(AttentionArgs a) {
     constexpr int CH = HD / 8;
     extern __shared__ __align__(128) unsigned char smem[];
     const uint32_t sQ = (uint32_t)__cvta_generic_to_shared(smem);
@@ -584,12 +588,46 @@ __global__ void __launch_bounds__(NTHREADS) attention_prefill_shared_kernel(Atte
     cluster_sync();                            // no block leaves while another may still read its weights
 }
 
+// Blocks a query tile and head.  More of them shorten the chain of key tiles and split O's columns, so that even one key tile is
+// faster with four; eight pay from five key tiles on (that many of them work in a round), and never more than find room at
+// once: two a multiprocessor where their shared memory allows it, and of clusters of four and eight about seven eighths
+// of that (the multiprocessors come in groups that such clusters do not fill).  Two blocks save less than their
+// barriers cost with heads of up to 64.  Microseconds with 1 / 2 / 4 / 8 blocks, T key tiles, P pairs of query tile and head:
+//   heads of 256  T 1, P 8     15.8 / 13.0 / 11.6 / 11.8      heads of 128  T 2, P 16    15.8 / 11.1 / 10.0 / 12.0
+//                 T 4, P 8     45.4 / 27.2 / 17.1 / 16.4                    T 4, P 16    27.0 / 18.4 / 11.6 / 13.6
+//                 T 5, P 8     55.0 / 35.2 / 23.8 / 17.4                    T 9, P 16    54.3 / 34.5 / 21.7 / 19.3
+//                 T 11, P 32    113 / 63.0 / 38.0 / 32.0                    T 9, P 64    55.0 / 35.0 / 24.9 / 42.6
+//                 T 11, P 40    113 / 63.1 / 40.6 / 57.7                    T 9, P 128   55.1 / 37.0 / 48.4 / 83.9
+//                 T 11, P 64    114 / 63.2 / 41.1 / 62.8      heads of 64   T 9, P 16    29.4 / 31.0 / 21.6 / 21.0
+//                 T 11, P 72    114 / 63.2 / 74.8 / 86.8                    T 9, P 64    29.6 / 31.7 / 27.7 / 51.1
+//                 T 11, P 144   115 / 68.5 / 115 / 149                      T 9, P 128   29.9 / 35.6 / 50.2 / 81.4
+// smem(runs): bytes of a block.  max_keys: the host's bound on the keys a query sees (0: not known); it and the rule change times only.
+template <typename Smem>
+int choose_runs(long long pairs, int head_dim, int max_keys, int sms, Smem smem) {
+    const int key_tiles = max_keys > 0 ? (max_keys + BN - 1) / BN : MAX_RUNS;
+    for (int runs = key_tiles > 4 ? MAX_RUNS : 4; runs > 1; runs /= 2) {
+        if (runs == 2 && head_dim <= 64) continue;
+        const long long slots = (long long)sms * std::min(2, 228 * 1024 / (smem(runs) + 1024));
+        if (pairs * runs <= (runs == 2 ? slots : slots * 7 / 8)) return runs;
+    }
+    return 1;
+}
+
+// f(HD, MODE) as integral constants: the widths and forms there are kernels for (softmax, sigmoid weights or a distance bias: kernels
+// of their own, so that the softmax kernels keep their registers).
+template <typename F>
+int by_form(int head_dim, bool sigmoid, bool rel, F f) {
+    auto mode = [&](auto hd) {
+        return sigmoid ? f(hd, std::integral_constant<int, 1>()) : rel ? f(hd, std::integral_constant<int, 2>()) : f(hd, std::integral_constant<int, 0>());
+    };
+    return head_dim <= 32 ? mode(std::integral_constant<int, 32>()) : head_dim <= 64 ? mode(std::integral_constant<int, 64>())
+           : head_dim <= 128 ? mode(std::integral_constant<int, 128>()) : mode(std::integral_constant<int, 256>());
+}
+
 template <int HD, int MODE>
 int launch_prefill_as(const AttentionArgs* a, cudaStream_t st) {
-    // Blocks a query tile: one where the query tiles alone fill the chip, else the most with which all blocks find room at once.
-    const long long blocks = (long long)a->n_tiles * a->n_heads;
-    int runs = 1;
-    while (runs < MAX_RUNS && blocks * 2 * runs <= 2LL * rdl_sm_count()) runs *= 2;
+    const int runs = choose_runs((long long)a->n_tiles * a->n_heads, a->head_dim, a->max_keys, rdl_sm_count(),
+                                 [&](int r) { return SharedLayout<HD, MODE>::total(a->head_dim, r); });
     if (runs == 1) {
         const int smem = (BM + 2 * BN) * HD * 2;
         static bool opted = false;
@@ -627,12 +665,6 @@ int launch_prefill_as(const AttentionArgs* a, cudaStream_t st) {
     return 0;
 }
 
-// softmax, sigmoid weights or a distance bias (kernels of their own, so that the softmax kernels keep their registers)
-template <int HD>
-int launch_prefill(const AttentionArgs* a, cudaStream_t st) {
-    return a->sigmoid_bias ? launch_prefill_as<HD, 1>(a, st) : (a->rel_bias ? launch_prefill_as<HD, 2>(a, st) : launch_prefill_as<HD, 0>(a, st));
-}
-
 }  // namespace
 
 extern "C" int rdl_attention_prefill(const AttentionArgs* a, void* stream) {
@@ -647,9 +679,11 @@ extern "C" int rdl_attention_prefill(const AttentionArgs* a, void* stream) {
                     ((uintptr_t)a->k_cache % 16 == 0) && ((uintptr_t)a->v_cache % 16 == 0) && ((uintptr_t)a->out % 4 == 0),
                 "attention_prefill: rows must start on 16-byte boundaries");
     if (a->n_tiles == 0 || a->n_tokens == 0) return 0;
-    cudaStream_t st = (cudaStream_t)stream;
-    if (a->head_dim <= 32) return launch_prefill<32>(a, st);
-    if (a->head_dim <= 64) return launch_prefill<64>(a, st);
-    if (a->head_dim <= 128) return launch_prefill<128>(a, st);
-    return launch_prefill<256>(a, st);
+    return by_form(a->head_dim, a->sigmoid_bias, a->rel_bias, [&](auto hd, auto mode) { return launch_prefill_as<hd.value, mode.value>(a, (cudaStream_t)stream); });
+}
+
+extern "C" int rdl_attention_prefill_blocks(long long pairs, int head_dim, int sigmoid, int max_keys, int sms) {
+    return by_form(head_dim, sigmoid != 0, false, [&](auto hd, auto mode) {
+        return choose_runs(pairs, head_dim, max_keys, sms, [&](int r) { return SharedLayout<hd.value, mode.value>::total(head_dim, r); });
+    });
 }

@@ -23,7 +23,7 @@ from concurrent.futures import ThreadPoolExecutor
 _PKG = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(_PKG, "csrc")
 LIB_NAME = "librdl_b200_kernels.so"
-ABI_VERSION = 21
+ABI_VERSION = 22
 
 # fast math is never enabled: the 32-bit path relies on exact tanhf/expf/sqrtf and plain FMA
 NVCC_FLAGS = ["-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
@@ -174,7 +174,7 @@ class AttentionArgs(ctypes.Structure):
         ("rope_cos", ctypes.c_void_p), ("rope_sin", ctypes.c_void_p), ("rotary_dim", ctypes.c_int), ("new_rows", ctypes.c_int),
         ("sinks", ctypes.c_void_p), ("sigmoid_bias", ctypes.c_void_p),
         ("chunk", ctypes.c_int), ("rel_bias", ctypes.c_void_p), ("rel_len", ctypes.c_int),
-        ("kv_share", ctypes.c_int),
+        ("kv_share", ctypes.c_int), ("max_keys", ctypes.c_int),
         ("wait_cycles", ctypes.c_longlong), ("test_extra_tx", ctypes.c_int),     # filled in by the launcher
     ]
 
@@ -394,6 +394,7 @@ _SIGNATURES = {
     "rdl_attention_plain": [ctypes.POINTER(AttentionArgs), _P],
     "rdl_attention_prefill": [ctypes.POINTER(AttentionArgs), _P],
     "rdl_attention_decode": [ctypes.POINTER(AttentionArgs), _P],
+    "rdl_attention_prefill_blocks": [_LL, _I, _I, _I, _I],
     "rdl_attention_prefill_tc": [ctypes.POINTER(AttentionArgs), _LL, _P],
     "rdl_embed_rows": [_P, _P, _I, _P, _F, _I, _I, _I, _P, _P, _I, _P, _I, _P],
     "rdl_norm_residual_norm": [_P, _I, _P, _P, _I, _F, _F, _P, _P, _P, _P, _P, _I, _F, _F, _P, _I, _I, _I, _P],

@@ -921,7 +921,7 @@ class AttentionBatch(NamedTuple):
     tile_seq: Optional[torch.Tensor] = None   # prefill: query tiles of PREFILL_QUERY_TILE rows
     tile_q0: Optional[torch.Tensor] = None
     n_tiles: int = 0
-    max_keys: int = 0          # decode: longest key run any token of the batch reads (window applied)
+    max_keys: int = 0          # longest key run any token of the batch reads (window applied); decode needs it, prefill is faster with it
 
 
 def _attention_args(q, q_stride, k_new, v_new, kv_stride, out, b: AttentionBatch, pages: Optional[KVPages],
@@ -1034,6 +1034,7 @@ def attention(q: torch.Tensor, b: AttentionBatch, pages: Optional[KVPages], *, n
     elif kind in ("prefill", "prefill_tc"):
         _need(b.tile_seq is not None and b.tile_q0 is not None, "attention: prefill needs query tiles")
         a.tile_seq, a.tile_q0, a.n_tiles = b.tile_seq.data_ptr(), b.tile_q0.data_ptr(), b.n_tiles
+        a.max_keys = b.max_keys
         if kind == "prefill_tc":
             # sequences that start at position 0, packed q/k/v rows, head_dim a multiple of 64
             _need(new_kv is not None and new_kv[0] is q, "attention: the tcgen05 prefill kernel reads packed q/k/v rows")

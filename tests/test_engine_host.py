@@ -226,3 +226,15 @@ def test_a_run_that_reads_another_runs_ring_sees_the_rows_of_earlier_steps(tmp_p
     engine.release(slot)
     slot = engine.new_sequence()
     close(torch.cat([engine.step([slot], [[t]], "all") for t in ids]), whole)
+
+
+def test_prompt_attention_blocks_follow_the_keys_and_the_room():
+    """How many blocks share a query tile and head: no more than a short prompt's keys can feed, no more than find room at once
+    (two a multiprocessor where their memory allows; clusters of four and eight leave an eighth of them empty)."""
+    from rust_deeplearning_b200.kernels import library
+    blocks = lambda pairs, hd, keys, sigmoid=0: library.load().rdl_attention_prefill_blocks(pairs, hd, sigmoid, keys, 148)
+    assert [blocks(8, 256, k) for k in (0, 1, 64, 256, 257, 8000)] == [8, 4, 4, 4, 8, 8]           # (0: not known)
+    assert [blocks(p, 256, 700) for p in (1, 32, 33, 64, 65, 148, 149, 10 ** 9)] == [8, 8, 4, 4, 2, 2, 1, 1]
+    assert [blocks(p, 256, 700, 1) for p in (16, 17, 32, 33, 74, 75)] == [8, 4, 4, 2, 2, 1]        # its memory leaves room for one
+    assert [blocks(p, 64, 700) for p in (32, 64, 65, 148)] == [8, 4, 1, 1]
+    assert [blocks(p, 16, 45) for p in (64, 65)] == [4, 1]
