@@ -38,7 +38,8 @@ __global__ void __launch_bounds__(256, RPT <= 8 ? 5 : (RPT == 16 ? 4 : (RPT == 3
     const int seq = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * DA_COLS;
     const int row0 = a.seq_start[seq], n = a.seq_start[seq + 1] - row0, slot = a.slots[seq];
     if (n <= 0) return;
-    const int first_pos = a.tok_pos[row0];   // (negative: a padding sequence of a fixed-size batch, which left its slot's state alone)
+    const int first_pos = a.tok_pos[row0];
+    if (first_pos < 0) return;               // a padding sequence of a fixed-size batch: its slot need not be one
     const int tid = threadIdx.x, j = tid & 31, r = tid >> 5, n_thr = blockDim.x;
     const int col = c0 + j;
     const bool col_ok = col < vdim;
@@ -71,7 +72,6 @@ __global__ void __launch_bounds__(256, RPT <= 8 ? 5 : (RPT == 16 ? 4 : (RPT == 3
         if (r == 0) v_in[b * DA_COLS + j] = a.silu ? silu_f(pv) : pv;
     };
     fetch(0);
-    if (first_pos < 0) return;
     stage(0);
     __syncthreads();
     for (int t = 0; t < n; ++t) {
@@ -136,9 +136,11 @@ __global__ void __launch_bounds__(8 * DS_GROUPS, 4) decay_step_kernel(DecayAtten
     rdl_grid_wait();
     rdl_grid_launch_dependents();
     const int seq = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * DS_COLS;
-    const int row0 = a.seq_start[seq], n = a.seq_start[seq + 1] - row0, slot = a.slots[seq];
+    // (as many rows as sequences: its row is most often the one of its number, whose position comes in the same trip)
+    const int row0 = a.seq_start[seq], n = a.seq_start[seq + 1] - row0, slot = a.slots[seq], pos_here = a.tok_pos[seq];
     if (n <= 0) return;
-    const int first_pos = a.tok_pos[row0];   // (negative: a padding sequence of a fixed-size batch, which left its slot's state alone)
+    const int first_pos = row0 == seq ? pos_here : a.tok_pos[row0];
+    if (first_pos < 0) return;               // a padding sequence of a fixed-size batch: its slot need not be one
     const int tid = threadIdx.x, r = tid / DS_GROUPS, n_thr = blockDim.x, i0 = r * RPT;
     const int col = c0 + (tid % DS_GROUPS) * 4;
     const bool col_ok = col < vdim;          // (vdim is a multiple of four)

@@ -258,6 +258,24 @@ def test_decay_attention_token_by_token(dtype, case):
     assert torch.equal(st2, st)
 
 
+@pytest.mark.parametrize("lens,pads", [([1, 1], 3), ([4, 1], 2)])           # the kernel of single-token steps, and the scan
+def test_decay_attention_leaves_the_slots_of_padding_sequences_alone(lens, pads):
+    """Sequences whose row stands at position -1 carry a slot that is no row of the state.  (The state is a part of a wider buffer,
+    so that slot -1 lies in memory of the test's own.)"""
+    rows, state, kw, _, _ = _decay_case(H=2, dim=64, vdim=32, lens=lens, past=[3, 0], rot_n=64, silu=False, k_scale=0.1, decays=[0.9, 0.99],
+                                        dtype=torch.float32, seed=61)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    T = sum(lens)
+    st = state.clone()
+    want = ops.decay_attention(rows, state=st, kind="scan", **kw)
+    wide = torch.full((state.shape[0] + 1, *state.shape[1:]), math.nan, device=DEV)
+    wide[1:] = state
+    padded = dict(kw, tok_pos=torch.cat([kw["tok_pos"], i32([-1] * pads)]), seq_start=torch.cat([kw["seq_start"], i32([T + 1 + i for i in range(pads)])]),
+                  slots=torch.cat([kw["slots"], i32([-1] * pads)]), n_seqs=len(lens) + pads)
+    got = ops.decay_attention(torch.cat([rows, rows[:pads]]), state=wide[1:], kind="scan", **padded)
+    assert torch.equal(got[:T], want) and torch.equal(wide[1:], st) and bool(torch.isnan(wide[0]).all())
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("case", [
     dict(H=2, dim=100, vdim=132, lens=[3, 1], past=[0, 4], rot_n=100, silu=True, k_scale=0.1, decays=[0.9, 0.99]),
