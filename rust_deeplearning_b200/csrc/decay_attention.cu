@@ -20,11 +20,11 @@
 
 __device__ __forceinline__ float silu_f(float z) { return z / (1.0f + expf(-z)); }
 
-// Left alone the compiler took 128 registers (two blocks a multiprocessor), and the state was asked for behind four trips to
-// memory in a row.  Four blocks (64 registers), everything that hangs on the sequence alone asked for at once: a
-// single-token step of 32 sequences of 16 heads of 128 x 128 (67 MB) took 21.0 us instead of 23.9.
+// A step's tokens one after the other, bound by the chain of them: a token's products, the sums over a block's slices, the
+// next one's vectors through shared memory.  The registers are left to the compiler (128 with 16 rows a thread): holding them to 64, for more blocks a multiprocessor, doubled the chain.  16 heads, one sequence of 300 float rows,
+// left alone / held: 128 x 128 321 / 601 us, 64 x 64 300 / 441 us, 32 x 32 235 / 309 us.
 template <typename T, int RPT>
-__global__ void __launch_bounds__(256, RPT <= 8 ? 5 : (RPT == 16 ? 4 : (RPT == 32 ? 2 : 1))) decay_scan_kernel(DecayAttentionArgs a) {
+__global__ void __launch_bounds__(256) decay_scan_kernel(DecayAttentionArgs a) {
     extern __shared__ float sm[];
     const int dim = a.dim, vdim = a.vdim;
     float* q_raw = sm;                       // [2][dim]
@@ -36,16 +36,15 @@ __global__ void __launch_bounds__(256, RPT <= 8 ? 5 : (RPT == 16 ? 4 : (RPT == 3
     rdl_grid_wait();
     rdl_grid_launch_dependents();
     const int seq = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * DA_COLS;
-    const int row0 = a.seq_start[seq], n = a.seq_start[seq + 1] - row0, slot = a.slots[seq];
+    const int row0 = a.seq_start[seq], n = a.seq_start[seq + 1] - row0;
     if (n <= 0) return;
-    const int first_pos = a.tok_pos[row0];
-    if (first_pos < 0) return;               // a padding sequence of a fixed-size batch: its slot need not be one
+    if (a.tok_pos[row0] < 0) return;         // a padding sequence of a fixed-size batch
     const int tid = threadIdx.x, j = tid & 31, r = tid >> 5, n_thr = blockDim.x;
     const int col = c0 + j;
     const bool col_ok = col < vdim;
     const int i0 = r * RPT;
     const float decay = a.decay[h];
-    float* S = a.state + (((long long)slot * a.n_heads + h) * dim) * vdim;
+    float* S = a.state + (((long long)a.slots[seq] * a.n_heads + h) * dim) * vdim;
     float s_reg[RPT];
 #pragma unroll
     for (int i = 0; i < RPT; ++i) s_reg[i] = (col_ok && i0 + i < dim) ? S[(long long)(i0 + i) * vdim + col] : 0.f;
@@ -78,7 +77,7 @@ __global__ void __launch_bounds__(256, RPT <= 8 ? 5 : (RPT == 16 ? 4 : (RPT == 3
         const int b = t & 1;
         if (t + 1 < n) fetch(t + 1);
         // q and k of this token as they enter the recurrence
-        const int pos = t == 0 ? first_pos : a.tok_pos[row0 + t];
+        const int pos = a.tok_pos[row0 + t];
         for (int i = tid; i < dim; i += n_thr) {
             float qv, kv;
             if (i < 2 * half) {
@@ -125,7 +124,7 @@ __global__ void __launch_bounds__(256, RPT <= 8 ? 5 : (RPT == 16 ? 4 : (RPT == 3
 // slice for four columns, in 16-byte accesses, so that a multiprocessor has 128 KB of state on its way instead of 64, and
 // every value of the token is fetched by the thread that needs it (one trip).  A block owns DS_COLS columns of a head.  The
 // slices, and the order of every sum, are those of the kernel above: the results are the same bits.
-// 32 sequences of 16 heads of 128 x 128: 21.0 -> 14.6 us (4.6 TB/s).
+// 32 sequences of 16 heads of 128 x 128 (67 MB of state), one call after the other: 19.8 us in the kernel above, 11.8 here.
 #define DS_GROUPS 16                   // groups of four columns
 #define DS_COLS (4 * DS_GROUPS)
 template <typename T, int RPT>
