@@ -452,8 +452,9 @@ __device__ __noinline__ bool few_candidates(int* out_tokens, int* host_tokens, c
     unsigned best = 0u;
 #pragma unroll
     for (int i = 0; i < CL_ITEMS; ++i) best = max(best, ordered_key(v[i]));
-    const bool at_top = best >= 0xff800000u;               // an infinity or a NaN
+    const unsigned undivided = best;
     best = ordered_key(key_value(best) / prm.temperature);
+    const bool at_top = max(undivided, best) >= 0xff800000u;      // an infinity or a NaN, or one after the division
     // A bound that k of the block's 1,024 largest-of-a-thread keys reach, and not many more: bit by bit from the top, until
     // the count is close enough.
     unsigned bound = 0u;
@@ -471,8 +472,8 @@ __device__ __noinline__ bool few_candidates(int* out_tokens, int* host_tokens, c
     parity ^= 1;
     if (best >= bound) {
         if (at_top) atomicAdd(&n_mine, FEW_CAP + 1);
-        // what is below this before the division is below the bound after it
-        const float scaled = key_value(bound) * prm.temperature, maybe = scaled - fabsf(scaled) * 1e-5f - 1e-37f;
+        // what is below this before the division is below the bound after it (whose last bit is that of a denormal at least)
+        const float scaled = key_value(bound) * prm.temperature, maybe = scaled - fabsf(scaled) * 1e-5f - 1e-37f - prm.temperature * 1.5e-45f;
 #pragma unroll
         for (int i = 0; i < CL_ITEMS; ++i) {
             if (!(v[i] >= maybe)) continue;
@@ -486,7 +487,8 @@ __device__ __noinline__ bool few_candidates(int* out_tokens, int* host_tokens, c
     cl_sync();                                             // every block's candidates lie in its shared memory
     unsigned n = 0u, from = 0u;
     for (int r = 0; r < n_blocks; ++r) n += cl_ld_u32(cl_map(&n_mine, r));
-    const bool few = bound > ordered_key(-INFINITY) && n <= (unsigned)FEW_CAP;
+    // (fewer than k: a temperature for which the line above is no number)
+    const bool few = bound > ordered_key(-INFINITY) && n >= (unsigned)prm.top_k && n <= (unsigned)FEW_CAP;
     unsigned* all_key = list + 2 * FEW_CAP;
     unsigned* all_idx = all_key + FEW_CAP;
     if (few && rank == 0) {

@@ -646,6 +646,25 @@ def test_sampling_of_few_candidates_and_rows_that_have_more(vocab):
             assert ops.sample(logits, **args).tolist() == ref.sample(logits, **args).tolist(), (top_k, top_p)
 
 
+@pytest.mark.parametrize("vocab", [300, 40000, 262144])
+def test_sampling_of_rows_that_are_not_for_few_candidates(vocab):
+    """Infinities and NaN at the top, before and after the division by the temperature, and temperatures that make every logit
+    equal: such rows go the way of a larger top-k, and their result here does not hang on k."""
+    logits = rnd((6, vocab), torch.float32, 62, 2.0)
+    logits[1, vocab // 2] = math.inf
+    logits[2] = -math.inf
+    logits[2, [7, vocab - 3]] = torch.tensor([math.nan, 30.0], device=DEV)
+    logits[3, ::5] = math.inf
+    logits[4, [3, 200, vocab - 1]] = 1e38                       # finite, infinite once divided by 1e-7
+    logits[5] = 1e38
+    for temperature, rows in ((0.9, [1, 2, 3]), (1e-7, [1, 2, 3, 4, 5]), (math.inf, [0, 5]), (3e38, [0])):
+        x = logits[rows].contiguous() * (1e-9 if temperature == 3e38 else 1.0)          # (every quotient rounds to zero there)
+        for top_p in (1.0, 0.9):
+            run = lambda k: ops.sample(x, temperature=temperature, seed=5, top_k=k, top_p=top_p).tolist()
+            want = run(257)
+            assert all(0 <= t < vocab for t in want) and [run(k) for k in (1, 40, 256)] == [want] * 3, (temperature, top_p)
+
+
 @pytest.mark.parametrize("vocab", [256, 40000])
 def test_sampling_takes_minus_zero_for_zero(vocab):
     """Logits that are +0 and -0 in turn are all equal: the thresholds of top-k and top-p (found on bit patterns)
