@@ -258,14 +258,22 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(int* __restrict_
 // 256,000 tokens, one row: 34 us plain, 92 us with top-k or top-p, 151 us with both (118 / 606 / 887 / 1,289 us
 // in the one-block kernel); two bits a round (three nested candidates) was no faster.
 //
-// With a top-k of up to FEW_TOP_K the rounds are not needed (few_candidates below): the k-th largest of a block's 1,024
+// With a small top-k the rounds are not needed (few_candidates below): the k-th largest of a block's 1,024
 // largest-of-a-thread values is a bound that at least k elements reach and that few others do, so the elements at or above
 // the highest block's bound - a few dozen of 256,000 - go to one block, which sorts them and does the rest alone.  What
-// bounds it is the row's one trip from L2 and two cluster barriers.  Rows with more candidates than a block sorts (long ties), with fewer
-// than k numbers above minus infinity, or with an infinity or NaN at the top take the rounds.
+// bounds it is the row's one trip from L2 and three cluster barriers.  Rows with more candidates than a block sorts (long ties), with fewer
+// than k numbers above minus infinity, or with an infinity or NaN at the top take the rounds after it, a trip of the row
+// and two barriers later.  Whether a call tries it is few_ok below; calls that cannot are a kernel without it, whose registers it would cost.
 // ---------------------------------------------------------------------------------------------
 constexpr int CL_THREADS = 1024, CL_ITEMS = 32, CL_PER_BLOCK = CL_THREADS * CL_ITEMS, CL_MAX_BLOCKS = 8;
 constexpr int FEW_TOP_K = 256, FEW_CAP = CL_THREADS;      // candidates one block sorts, a thread each
+
+// Whether a top-k brings no more candidates than one block sorts: about k of every block.  256,000 tokens (eight blocks), one row,
+// with the shortcut / without: k = 40 17.2 / 71 us, 104 22.5 / 84, 120 23.7 / 80 (64 rows, some of which have more: 172 / 386),
+// 256 92 / 80.  A row of 30 finite logits, which takes the rounds after it: 130 us / 105.
+static bool few_ok(int top_k, int vocab, int n_blocks) {
+    return top_k > 0 && top_k < vocab && top_k <= FEW_TOP_K && top_k * n_blocks <= FEW_CAP - 64;
+}
 
 __device__ __forceinline__ uint32_t cl_rank() {
     uint32_t r;
@@ -425,7 +433,7 @@ __device__ __forceinline__ int first_beyond(const float* mass, int n, float targ
     return found;
 }
 
-// Top-k of up to FEW_TOP_K (see above).  false, the same in every block of the cluster: the row is not one for it, nothing was
+// A small top-k (see above).  false, the same in every block of the cluster: the row is not one for it, nothing was
 // written.  `list`: at least 6 * FEW_CAP words of shared memory.
 __device__ __noinline__ bool few_candidates(int* out_tokens, int* host_tokens, const float* src, int row, int vocab, const SamplingArgs& prm,
                                const unsigned long long* row_stream, const int* row_step, int rank, int n_blocks, unsigned* list,
@@ -575,6 +583,8 @@ __device__ __noinline__ bool few_candidates(int* out_tokens, int* host_tokens, c
     return true;
 }
 
+// FEW: the shortcut for a small top-k is tried first.
+template <bool FEW>
 __global__ void __launch_bounds__(CL_THREADS, 1) sample_cluster_kernel(int* __restrict__ out_tokens, int* __restrict__ host_tokens, const float* __restrict__ logits,
                                                                        int vocab, SamplingArgs prm,
                                                                        const unsigned long long* __restrict__ row_stream,
@@ -617,9 +627,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) sample_cluster_kernel(int* __re
         cl_sync();
         src = w;
     }
-    if (prm.top_k > 0 && prm.top_k < vocab && prm.top_k <= FEW_TOP_K &&
-        few_candidates(out_tokens, host_tokens, src, row, vocab, prm, row_stream, row_step, rank, n_blocks, keys, &xch, parity))
-        return;
+    if (FEW && few_candidates(out_tokens, host_tokens, src, row, vocab, prm, row_stream, row_step, rank, n_blocks, keys, &xch, parity)) return;
     float e[CL_ITEMS];                                        // the scaled logits first, their exponentials later
     float mx = -INFINITY;
 #pragma unroll
@@ -781,9 +789,11 @@ extern "C" int rdl_sample(int* out_tokens, int* host_tokens, const float* logits
         int n_blocks = 1;
         while (n_blocks * CL_PER_BLOCK < vocab) n_blocks *= 2;
         const size_t smem = (size_t)CL_ITEMS * CL_THREADS * sizeof(unsigned);
+        const bool few = few_ok(prm->top_k, vocab, n_blocks);
         static bool opted = false;
         if (!opted) {
-            RDL_CUDA(cudaFuncSetAttribute(sample_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "sample");
+            RDL_CUDA(cudaFuncSetAttribute(sample_cluster_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "sample");
+            RDL_CUDA(cudaFuncSetAttribute(sample_cluster_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "sample");
             opted = true;
         }
         cudaLaunchConfig_t cfg = {};
@@ -799,8 +809,8 @@ extern "C" int rdl_sample(int* out_tokens, int* host_tokens, const float* logits
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = g_rdl_programmatic_launch ? 2 : 1;
-        RDL_CHECK_EX(cudaLaunchKernelEx(&cfg, sample_cluster_kernel, out_tokens, host_tokens, logits, vocab, *prm, row_stream, row_step, history,
-                                        history_start, work, n_blocks), "sample");
+        RDL_CHECK_EX(cudaLaunchKernelEx(&cfg, few ? sample_cluster_kernel<true> : sample_cluster_kernel<false>, out_tokens, host_tokens, logits, vocab, *prm,
+                                        row_stream, row_step, history, history_start, work, n_blocks), "sample");
         return 0;
     }
     RDL_CHECK_EX(rdl_launch(sample_kernel, dim3(n_rows), dim3(SAMPLE_THREADS), 0, (cudaStream_t)stream, out_tokens, host_tokens, logits, vocab,
