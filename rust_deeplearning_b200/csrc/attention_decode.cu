@@ -604,12 +604,7 @@ int launch_decode_as(const AttentionArgs* a, cudaStream_t st) {
     if (runs > smem) smem = runs;
     RDL_REQUIRE(smem <= 200 * 1024, "attention_decode: page_size %d x head_dim %d needs %d bytes of shared memory, limit is 204800",
                 a->page_size, a->head_dim, smem);
-    static int granted = 32 * 1024;      // above this the kernel (which also has a few KB of static shared memory) opts in
-    if (smem > granted) {
-        RDL_CUDA(cudaFuncSetAttribute(attention_decode_kernel<HD, EXACT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
-                 "attention_decode");
-        granted = smem;
-    }
+    RDL_CUDA((rdl_allow_shared<attention_decode_kernel<HD, EXACT, MODE>>(smem)), "attention_decode");
     dim3 grid(a->max_splits, a->n_kv_heads, a->n_tokens);
     AttentionArgs b = *a;
     b.wait_cycles = rdl_wait_cycles_for(RDL_FAULT_ATTENTION_DECODE);

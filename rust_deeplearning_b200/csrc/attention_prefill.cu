@@ -630,24 +630,14 @@ int launch_prefill_as(const AttentionArgs* a, cudaStream_t st) {
                                  [&](int r) { return SharedLayout<HD, MODE>::total(a->head_dim, r); });
     if (runs == 1) {
         const int smem = (BM + 2 * BN) * HD * 2;
-        static bool opted = false;
-        if (smem > 48 * 1024 && !opted) {
-            RDL_CUDA(cudaFuncSetAttribute(attention_prefill_kernel<HD, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
-                     "attention_prefill");
-            opted = true;
-        }
+        RDL_CUDA((rdl_allow_shared<attention_prefill_kernel<HD, MODE>>(smem)), "attention_prefill");
         dim3 grid(a->n_tiles, a->n_heads);
         RDL_CHECK_EX(rdl_launch(attention_prefill_kernel<HD, MODE>, grid, dim3(NTHREADS), (size_t)smem, st, *a), "attention_prefill");
         return 0;
     }
     using L = SharedLayout<HD, MODE>;
-    static bool opted = false;
-    if (!opted) {
-        const int most = std::max(std::max(L::total(HD, 2), L::total(HD, 4)), L::total(HD, 8));
-        RDL_CUDA(cudaFuncSetAttribute(attention_prefill_shared_kernel<HD, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, most),
-                 "attention_prefill");
-        opted = true;
-    }
+    const int smem = L::total(a->head_dim, runs);
+    RDL_CUDA((rdl_allow_shared<attention_prefill_shared_kernel<HD, MODE>>(smem)), "attention_prefill");
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -657,7 +647,7 @@ int launch_prefill_as(const AttentionArgs* a, cudaStream_t st) {
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.gridDim = dim3((unsigned)(a->n_tiles * runs), (unsigned)a->n_heads);
     cfg.blockDim = dim3(NTHREADS);
-    cfg.dynamicSmemBytes = (size_t)L::total(a->head_dim, runs);
+    cfg.dynamicSmemBytes = (size_t)smem;
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = g_rdl_programmatic_launch ? 2 : 1;

@@ -447,11 +447,7 @@ int make_map(CUtensorMap* map, const void* ptr, long long rows, long long cols, 
 
 template <int DB, bool REL>
 int launch_tc_as(dim3 grid, int smem, cudaStream_t st, const CUtensorMap& map_q, const CUtensorMap& map_kv, const TcAttnArgs& t) {
-    static int granted = 0;
-    if (smem > granted) {
-        RDL_CUDA(cudaFuncSetAttribute(attention_tc_kernel<DB, REL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "attention_prefill_tc");
-        granted = smem;
-    }
+    RDL_CUDA((rdl_allow_shared<attention_tc_kernel<DB, REL>>(smem)), "attention_prefill_tc");
     RDL_CHECK_EX(rdl_launch(attention_tc_kernel<DB, REL>, grid, dim3(ATC_THREADS), (size_t)smem, st, map_q, map_kv, t), "attention_prefill_tc");
     return 0;
 }

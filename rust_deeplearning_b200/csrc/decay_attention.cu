@@ -672,11 +672,7 @@ extern "C" int rdl_decay_attention_chunked(const DecayAttentionArgs* a, void* wo
     const int qs = a->dim + DC_PAD, vs = DC_COLS + DC_PAD;
     const size_t smem_u = (size_t)(DC_CHUNK * qs + DC_CHUNK * vs) * 2;
     const size_t smem_o = (size_t)(2 * DC_CHUNK * qs + DC_CHUNK * vs + 2 * a->dim * vs) * 2;
-    static bool opted = false;
-    if (!opted) {
-        RDL_CUDA(cudaFuncSetAttribute(decay_chunk_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024), "decay_attention_chunked");
-        opted = true;
-    }
+    RDL_CUDA(rdl_allow_shared<decay_chunk_kernel<true>>(100 * 1024), "decay_attention_chunked");
     cudaStream_t st = (cudaStream_t)stream;
     const dim3 grid(max_chunks, a->n_heads, (a->vdim + DC_COLS - 1) / DC_COLS);
     // 16-byte loads where every head starts on a 16-byte boundary and the rotated half is a whole number of them

@@ -304,11 +304,7 @@ template <typename T, int RPS>
 int dc_launch(const RecurrenceArgs* a, float* records, int max_groups, cudaStream_t st) {
     using R = DcRecord<RPS>;
     const size_t smem = (size_t)DC_STAGES * R::STAGE * sizeof(float);
-    static bool opted = false;
-    if (!opted) {
-        RDL_CUDA(cudaFuncSetAttribute(dc_scan_kernel<RPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "delta_rule_chunked");
-        opted = true;
-    }
+    RDL_CUDA((rdl_allow_shared<dc_scan_kernel<RPS>>(smem)), "delta_rule_chunked");
     RDL_CHECK_EX(rdl_launch(dc_record_kernel<T, RPS>, dim3(max_groups, a->n_heads), dim3(128), 0, st, *a, records), "delta_rule_chunked (records)");
     RDL_CHECK_EX(rdl_launch(dc_scan_kernel<RPS>, dim3(a->n_seqs, a->n_heads, (a->vdim + DC_COLS - 1) / DC_COLS), dim3(DC_THREADS), smem, st, *a,
                             (const float*)records), "delta_rule_chunked (scan)");

@@ -301,13 +301,7 @@ extern "C" int rdl_norm_residual_norm(const void* x, int x_dtype, const int* row
     const size_t smem = (size_t)hidden * sizeof(float);
     RDL_REQUIRE(smem <= 200 * 1024, "norm: hidden size %d needs %zu bytes of shared memory, limit is 204800", hidden, smem);
     if (n_rows == 0) return 0;
-    if (smem > 48 * 1024) {
-        static size_t granted = 0;  // largest size already opted in
-        if (smem > granted) {
-            RDL_CUDA(cudaFuncSetAttribute(norm_residual_norm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "norm");
-            granted = smem;
-        }
-    }
+    RDL_CUDA(rdl_allow_shared<norm_residual_norm_kernel>((int)smem), "norm");
     NormArgs a{x, x_dtype, row_index, w1, w1_dtype, eps1, off1, (const float*)res_f32, (float*)res_out_f32, add_rows, add_vec, w2, w2_dtype, eps2, off2, y, y_dtype, hidden};
     const int threads = hidden >= 2048 ? 512 : (hidden >= 512 ? 256 : 128);
     RDL_CHECK_EX(rdl_launch(norm_residual_norm_kernel, dim3(n_rows), dim3(threads), smem, (cudaStream_t)stream, a), "norm_residual_norm");

@@ -170,12 +170,8 @@ cudaError_t launch_few(float* out, const float* x, const float* w, int M, int N,
     constexpr int FIT = (224 * 1024 - 2 * RUNS * MT * ROWS * 4) / (RUNS * STAGE_BYTES), STAGES = FIT > 10 ? 10 : FIT;
     static_assert(STAGES >= 3, "a ring of three chunks at least");
     constexpr size_t smem = (size_t)RUNS * STAGES * STAGE_BYTES;
-    static bool opted = false;
-    if (!opted) {
-        const cudaError_t e = cudaFuncSetAttribute(gemm_f32_few_kernel<ROWS, MT, STAGES, ALIGNED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        opted = true;
-    }
+    const cudaError_t e = rdl_allow_shared<gemm_f32_few_kernel<ROWS, MT, STAGES, ALIGNED>>((int)smem);
+    if (e != cudaSuccess) return e;
     const int tiles = (N + ROWS - 1) / ROWS, sms = rdl_sm_count();
     return rdl_launch(gemm_f32_few_kernel<ROWS, MT, STAGES, ALIGNED>, dim3(tiles < sms ? tiles : sms), dim3(RUNS * 32), smem, st, out, x, w, M, N, K);
 }
@@ -327,12 +323,8 @@ template <int TM, bool SHARED, bool ALIGNED>
 cudaError_t launch_tile(float* out, const float* x, const float* w, int M, int N, int K, cudaStream_t st) {
     constexpr int BM = 16 * TM;
     constexpr size_t smem = (size_t)(tile_stages(TM) * (BM + BN) * PITCH + BM * BN) * 4;
-    static bool opted = false;
-    if (!opted) {
-        const cudaError_t e = cudaFuncSetAttribute(gemm_f32_tile_kernel<TM, SHARED, ALIGNED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        opted = true;
-    }
+    const cudaError_t e = rdl_allow_shared<gemm_f32_tile_kernel<TM, SHARED, ALIGNED>>((int)smem);
+    if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((N + BN - 1) / BN, (M + BM - 1) / BM, SHARED ? RUNS : 1);
     cfg.blockDim = dim3(256);

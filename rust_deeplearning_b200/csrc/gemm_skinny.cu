@@ -423,14 +423,9 @@ template <int NT, bool GATED, int KU, int MODE>
 void launch_stream_ku(const SkinnyArgs& a, int* status, cudaStream_t st) {
     constexpr int smem_max = 2 * st_stages(KU) * st_tile_bytes(KU);
     static_assert(2 * st_stages(KU) <= ST_MAX_STAGES, "the ring's barriers");
-    static bool opted = false;
-    static int sms = 0;
-    if (!opted) {
-        g_launch_error = cudaFuncSetAttribute(gemm_stream_kernel<NT, GATED, KU, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
-        if (g_launch_error != cudaSuccess) return;
-        sms = rdl_sm_count();
-        opted = true;
-    }
+    g_launch_error = rdl_allow_shared<gemm_stream_kernel<NT, GATED, KU, MODE>>(smem_max);
+    if (g_launch_error != cudaSuccess) return;
+    const int sms = rdl_sm_count();
     // What counts is the bytes a multiprocessor has in flight: two blocks with three tiles each, or, where
     // the output is so narrow that there is at most one block a multiprocessor, one block with twice as many.
     const int units = (a.N + (GATED ? 8 : ROWS) - 1) / (GATED ? 8 : ROWS);

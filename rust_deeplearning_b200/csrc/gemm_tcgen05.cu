@@ -563,11 +563,7 @@ int launch_tc(const CUtensorMap& mx, const CUtensorMap& mw, const TcArgs& a, cud
     constexpr int NB = GATED ? 2 : 1;
     constexpr int STAGES = MT == 2 ? 3 : 4;
     const int smem = STAGES * (MT * BM * BK * 2 + NB * BN * BK * 2) + EPI_WARPS * EPI_STAGE_BYTES + 1024;
-    static bool opted = false;
-    if (!opted) {
-        RDL_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<BN, GATED, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "gemm_tc");
-        opted = true;
-    }
+    RDL_CUDA((rdl_allow_shared<gemm_tc_kernel<BN, GATED, MT>>(smem)), "gemm_tc");
     const long long tiles = (long long)((a.N + BN - 1) / BN) * ((a.M + MT * BM - 1) / (MT * BM));
     RDL_REQUIRE(tiles <= 0x7fffffffLL, "gemm_tc: %lld tiles exceed the grid limit", tiles);
     dim3 grid((unsigned)tiles);
@@ -579,18 +575,10 @@ template <bool GATED, int NACC>
 int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const TcArgs& a, cudaStream_t st) {
     constexpr int OUT_BN = GATED ? PAIR_BN / 2 : PAIR_BN;
     const int smem = PAIR_STAGES * (BM * BK * 2 + (PAIR_BN / 2) * BK * 2) + EPI_WARPS * EPI_STAGE_BYTES + 1024;
-    static bool opted = false;
-    if (!opted) {
-        RDL_CUDA(cudaFuncSetAttribute(gemm_tc_pair_kernel<GATED, NACC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "gemm_tc");
-        opted = true;
-    }
+    RDL_CUDA((rdl_allow_shared<gemm_tc_pair_kernel<GATED, NACC>>(smem)), "gemm_tc");
     const long long tiles = (long long)((a.N + OUT_BN - 1) / OUT_BN) * ((a.M + 2 * BM - 1) / (2 * BM));
     RDL_REQUIRE(tiles <= 0x3fffffffLL, "gemm_tc: %lld tiles are too many", tiles);
-    static int pairs_that_fit = 0;             // one block per multiprocessor: half as many pairs
-    if (!pairs_that_fit) {
-        const int sms = rdl_sm_count();
-        pairs_that_fit = sms / 2 > 0 ? sms / 2 : 1;
-    }
+    const int pairs_that_fit = rdl_sm_count() > 1 ? rdl_sm_count() / 2 : 1;      // one block per multiprocessor: half as many pairs
     const int pairs = tiles < pairs_that_fit ? (int)tiles : pairs_that_fit;
     RDL_CHECK_EX(rdl_launch(gemm_tc_pair_kernel<GATED, NACC>, dim3((unsigned)(2 * pairs)), dim3(PAIR_THREADS), (size_t)smem, st, mx, mw, a), "gemm_tc");
     return 0;

@@ -348,11 +348,7 @@ __global__ void __launch_bounds__(128) latent_decode_merge_kernel(LatentDecodeAr
 
 template <int NP, bool FULL>
 int launch_latent_decode_form(const LatentDecodeArgs& a, dim3 grid, size_t smem, cudaStream_t st) {
-    static bool opted = false;
-    if (!opted) {
-        RDL_CUDA(cudaFuncSetAttribute(latent_decode_kernel<NP, FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024), "latent_decode");
-        opted = true;
-    }
+    RDL_CUDA((rdl_allow_shared<latent_decode_kernel<NP, FULL>>(227 * 1024)), "latent_decode");
     RDL_CHECK_EX(rdl_launch(latent_decode_kernel<NP, FULL>, grid, dim3(LD_THREADS), smem, st, a), "latent_decode");
     return 0;
 }

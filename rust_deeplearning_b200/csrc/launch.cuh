@@ -19,6 +19,8 @@
 
 #include <utility>
 
+#include "per_device.h"
+
 // 1: launches carry the programmatic-serialization attribute.  Set through rdl_set_programmatic_launch.
 extern int g_rdl_programmatic_launch;
 
@@ -35,6 +37,16 @@ inline cudaError_t rdl_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
     cfg.attrs = attr;
     cfg.numAttrs = g_rdl_programmatic_launch ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+// Lets KERNEL take up to `bytes` of dynamic shared memory on the current device (the driver is asked where that is more than before).
+template <auto KERNEL>
+inline cudaError_t rdl_allow_shared(int bytes) {
+    static RdlRaisedPerDevice raised;
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    return (cudaError_t)raised.run(dev, bytes, [&] { return (int)cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); });
 }
 
 __device__ __forceinline__ void rdl_grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

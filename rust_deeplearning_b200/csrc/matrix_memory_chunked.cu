@@ -409,11 +409,7 @@ extern "C" int rdl_matrix_memory_chunked(const MatrixMemoryArgs* a, void* work, 
     const int qs = a->dim + CM_PAD, vs = MMC_COLS + CM_PAD;
     const size_t smem_u = (size_t)(CM_CHUNK * qs + 2 * CM_CHUNK * vs) * 2;
     const size_t smem_o = (size_t)(2 * CM_CHUNK * qs + CM_CHUNK * vs + 2 * a->dim * vs) * 2;
-    static bool opted = false;
-    if (!opted) {
-        RDL_CUDA(cudaFuncSetAttribute(mm_chunk_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024), "matrix_memory_chunked");
-        opted = true;
-    }
+    RDL_CUDA(rdl_allow_shared<mm_chunk_kernel<true>>(112 * 1024), "matrix_memory_chunked");
     cudaStream_t st = (cudaStream_t)stream;
     const dim3 grid(max_chunks, a->n_heads, (a->vdim + MMC_COLS - 1) / MMC_COLS);
     RDL_CHECK_EX(rdl_launch(mm_chunk_kernel<false>, grid, dim3(MMC_THREADS), smem_u, st, *a, w), "matrix_memory_chunked (chunk states)");

@@ -790,12 +790,7 @@ extern "C" int rdl_sample(int* out_tokens, int* host_tokens, const float* logits
         while (n_blocks * CL_PER_BLOCK < vocab) n_blocks *= 2;
         const size_t smem = (size_t)CL_ITEMS * CL_THREADS * sizeof(unsigned);
         const bool few = few_ok(prm->top_k, vocab, n_blocks);
-        static bool opted = false;
-        if (!opted) {
-            RDL_CUDA(cudaFuncSetAttribute(sample_cluster_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "sample");
-            RDL_CUDA(cudaFuncSetAttribute(sample_cluster_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "sample");
-            opted = true;
-        }
+        RDL_CUDA(few ? rdl_allow_shared<sample_cluster_kernel<true>>((int)smem) : rdl_allow_shared<sample_cluster_kernel<false>>((int)smem), "sample");
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(n_blocks, n_rows);
         cfg.blockDim = dim3(CL_THREADS);

@@ -312,11 +312,7 @@ extern "C" int rdl_state_space_chunked(const RecurrenceArgs* a, void* work, long
     const int qs = a->dim + CM_PAD, vs = SSC_COLS + CM_PAD;
     const size_t smem_u = (size_t)(CM_CHUNK * qs + 2 * CM_CHUNK * vs) * 2;
     const size_t smem_o = (size_t)(2 * CM_CHUNK * qs + 2 * CM_CHUNK * vs + 2 * a->dim * vs) * 2;
-    static bool opted = false;
-    if (!opted) {
-        RDL_CUDA(cudaFuncSetAttribute(ssc_chunk_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024), "state_space_chunked");
-        opted = true;
-    }
+    RDL_CUDA(rdl_allow_shared<ssc_chunk_kernel<true>>(112 * 1024), "state_space_chunked");
     cudaStream_t st = (cudaStream_t)stream;
     const dim3 grid(max_chunks, a->n_heads, (a->vdim + SSC_COLS - 1) / SSC_COLS);
     RDL_CHECK_EX(rdl_launch(ssc_chunk_kernel<false>, grid, dim3(SSC_THREADS), smem_u, st, *a, totals, states), "state_space_chunked (chunk states)");

@@ -238,3 +238,55 @@ def test_prompt_attention_blocks_follow_the_keys_and_the_room():
     assert [blocks(p, 256, 700, 1) for p in (16, 17, 32, 33, 74, 75)] == [8, 4, 4, 2, 2, 1]        # its memory leaves room for one
     assert [blocks(p, 64, 700) for p in (32, 64, 65, 148)] == [8, 4, 1, 1]
     assert [blocks(p, 16, 45) for p in (64, 65)] == [4, 1]
+
+
+def test_what_a_device_needs_raised_is_raised_on_every_device(tmp_path):
+    """`csrc/per_device.h`, which the launchers keep the opt-in to more shared memory with: asked for once a device and size, again
+    where it failed, never lowered, and by several threads."""
+    import os
+    import shutil
+    import subprocess
+    from rust_deeplearning_b200.kernels import library
+    src = tmp_path / "t.cpp"
+    src.write_text(r"""
+#include "per_device.h"
+#include <cstdio>
+#include <thread>
+#include <vector>
+int main() {
+    RdlRaisedPerDevice r;
+    int calls = 0, result = 0;
+    auto f = [&] { ++calls; return result; };
+    auto want = [&](int device, int value, int status, int n, int line) {
+        calls = 0;
+        const int e = r.run(device, value, f);
+        if (e != status || calls != n) { std::printf("line %d: %d, %d calls\n", line, e, calls); std::exit(1); }
+    };
+    want(0, 100, 0, 1, __LINE__);
+    want(0, 100, 0, 0, __LINE__);
+    want(1, 100, 0, 1, __LINE__);      // another device has not been asked
+    want(0, 50, 0, 0, __LINE__);
+    want(0, 200, 0, 1, __LINE__);
+    want(1, 100, 0, 0, __LINE__);
+    result = 7;
+    want(63, 10, 7, 1, __LINE__);
+    want(63, 10, 7, 1, __LINE__);      // a failure is not remembered
+    result = 0;
+    want(63, 10, 0, 1, __LINE__);
+    want(64, 10, 0, 1, __LINE__);
+    want(64, 10, 0, 1, __LINE__);
+    int set = 0;                       // threads with other sizes: the last one set is the largest
+    std::vector<std::thread> ts;
+    for (int t = 1; t <= 8; ++t) ts.emplace_back([&, t] { for (int i = 0; i < 1000; ++i) r.run(5, t * 1000 + i, [&] { set = t * 1000 + i; return 0; }); });
+    for (auto& t : ts) t.join();
+    if (set != 8999) { std::printf("ended at %d\n", set); return 1; }
+    return 0;
+}
+""")
+    exe = tmp_path / "t"
+    subprocess.run([shutil.which("g++") or "c++", "-std=c++17", "-O1", "-pthread", "-I", library.CSRC, "-include", "cstdlib", str(src), "-o", str(exe)], check=True)
+    done = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert done.returncode == 0, done.stdout
+    for name in os.listdir(library.CSRC):       # nobody keeps such a thing once a process
+        text = open(os.path.join(library.CSRC, name)).read()
+        assert name == "launch.cuh" or "cudaFuncSetAttribute" not in text, name
