@@ -11,7 +11,7 @@ extern "C" {
 #define RDL_ACT_SILU 1
 #define RDL_ACT_SWISH_LIMIT 2   // min(g, L) sigmoid(1.702 min(g, L)) (clamp(u, -L, L) + 1), L a parameter
 
-#define RDL_ABI_VERSION 22
+#define RDL_ABI_VERSION 23
 
 const char* rdl_last_error(void);
 int rdl_abi_version(void);
@@ -220,7 +220,7 @@ int rdl_norm_shift(const float* x, const void* w, int w_dtype, float eps, const 
 // sequence's last taps - 1 inputs.  in: rows with a stride of their own; out dense [rows][channels]; bias optional.
 int rdl_short_conv(const void* in, long long in_stride, int dtype, int channels, int taps, const void* w, int w_dtype,
                    const void* bias, int silu, float* state, const int* tok_seq, const int* tok_pos, const int* seq_start,
-                   const int* slots, void* out, int n_rows, void* stream);
+                   const int* slots, void* out, int n_rows, int n_seqs, void* stream);
 // res[t, i] += sigmoid(gates[t, i] + bias_a[i]) a[t, i] + sigmoid(gates[t, width + i] + bias_b[i]) (b1[t, i] + b2[t, i]), in float;
 // b1 NULL: the first term only; b2 optional
 int rdl_gated_residual_add(float* res, const void* gates, long long gates_stride, const void* bias_a, const void* bias_b,

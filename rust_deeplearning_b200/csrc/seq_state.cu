@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(128) short_conv_kernel(const T* __restrict__ i
 
 // Four taps over many rows (a prompt): a thread takes 16 bytes of channels and four rows, whose seven inputs it loads once; the
 // kernel above loads two bytes at a time and every input four times.  Every output goes through the same operations.
-// Four prompts (3,400 rows) with two such layers and 16 single-token steps: 9.70 -> 9.51 ms.
+// Four prompts (3,400 rows) with two such layers and 16 single-token steps: 9.70 -> 9.51 ms; the rule at the launch has more.
 constexpr int CONV_RUN = 4;
 template <typename T>
 __global__ void __launch_bounds__(128) short_conv4_rows_kernel(const T* __restrict__ in, long long in_stride, int n_rows, int channels,
@@ -409,7 +409,7 @@ extern "C" int rdl_norm_shift(const float* x, const void* w, int w_dtype, float 
 
 extern "C" int rdl_short_conv(const void* in, long long in_stride, int dtype, int channels, int taps, const void* w, int w_dtype,
                               const void* bias, int silu, float* state, const int* tok_seq, const int* tok_pos, const int* seq_start,
-                              const int* slots, void* out, int n_rows, void* stream) {
+                              const int* slots, void* out, int n_rows, int n_seqs, void* stream) {
     RDL_REQUIRE(rdl_valid_dtype(dtype) && rdl_valid_dtype(w_dtype), "short_conv: bad dtype");
     RDL_REQUIRE(in && w && tok_seq && tok_pos && seq_start && slots && out && channels > 0 && in_stride >= channels && n_rows >= 0,
                 "short_conv: bad arguments");
@@ -420,8 +420,12 @@ extern "C" int rdl_short_conv(const void* in, long long in_stride, int dtype, in
     const dim3 grid(n_rows, (channels + 127) / 128), block(128);
     cudaStream_t st = (cudaStream_t)stream;
     const int piece = dtype == RDL_BF16 ? 8 : 4;
-    // (few rows: there the form above, a thread a channel, has more threads for the rows that read the slot)
-    if (n_rows >= 512 && taps == 4 && w_dtype == dtype && channels % piece == 0 && in_stride % piece == 0 && aligned16(in) && aligned16(w) && aligned16(out)) {
+    // Runs of four rows where there are many and most are not a sequence's first ones, which one thread takes for eight channels one
+    // after the other.  Microseconds, a thread a channel / runs of four, rows in sequences of L:
+    //   2,304 channels   512 rows    L 1 20 / 40    L 4 14 / 18    L 8 15 / 16    L 32 16 / 13    one 15 / 11       256 rows, one 10 / 11
+    //                    4,096 rows  L 1 150 / 216  L 4 82 / 79    L 8 82 / 55    L 32 84 / 38    one 82 / 30
+    //   6,144 channels   512 rows    L 1 46 / 77    L 4 30 / 31    L 8 31 / 24    L 32 32 / 19    one 32 / 16
+    if (n_rows >= 512 && n_rows >= 8LL * n_seqs && taps == 4 && w_dtype == dtype && channels % piece == 0 && in_stride % piece == 0 && aligned16(in) && aligned16(w) && aligned16(out)) {
         const dim3 runs((n_rows + CONV_RUN - 1) / CONV_RUN, (channels / piece + 127) / 128);
         if (dtype == RDL_BF16)
             RDL_CHECK_EX(rdl_launch(short_conv4_rows_kernel<__nv_bfloat16>, runs, block, 0, st, (const __nv_bfloat16*)in, in_stride, n_rows, channels,

@@ -23,7 +23,7 @@ from concurrent.futures import ThreadPoolExecutor
 _PKG = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(_PKG, "csrc")
 LIB_NAME = "librdl_b200_kernels.so"
-ABI_VERSION = 22
+ABI_VERSION = 23
 
 # fast math is never enabled: the 32-bit path relies on exact tanhf/expf/sqrtf and plain FMA
 NVCC_FLAGS = ["-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
@@ -412,7 +412,7 @@ _SIGNATURES = {
     "rdl_gate_mul": [_P, _LL, _P, _LL, _P, _LL, _I, _I, _I, _I, _P],
     "rdl_group_norm_gate": [_P, _I, _P, _I, _I, _I, _P, _I, _F, _P, _LL, _I, _I, _I, _P],
     "rdl_norm_shift": [_P, _P, _I, _F, _P, _I, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _P],
-    "rdl_short_conv": [_P, _LL, _I, _I, _I, _P, _I, _P, _I, _P, _P, _P, _P, _P, _P, _I, _P],
+    "rdl_short_conv": [_P, _LL, _I, _I, _I, _P, _I, _P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _P],
     "rdl_gated_residual_add": [_P, _P, _LL, _P, _P, _I, _P, _P, _P, _I, _I, _I, _P],
     "rdl_activation_inplace": [_P, _I, _LL, _I, _P],
     "rdl_recurrence_scan": [ctypes.POINTER(RecurrenceArgs), _P],

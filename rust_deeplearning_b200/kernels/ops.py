@@ -1561,7 +1561,7 @@ def short_conv(rows: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Te
     out = torch.empty((T, C), dtype=rows.dtype, device=rows.device)
     library.check(library.load().rdl_short_conv(_ptr(rows), rows.stride(0), _dtype_code(rows), C, taps, _ptr(weight), _dtype_code(weight),
                                                 _ptr(bias), int(bool(silu)), _ptr(state) if taps > 1 else None, _ptr(tok_seq),
-                                                _ptr(tok_pos), _ptr(seq_start), _ptr(slots), _ptr(out), T, _stream(rows)))
+                                                _ptr(tok_pos), _ptr(seq_start), _ptr(slots), _ptr(out), T, seq_start.numel() - 1, _stream(rows)))
     return out
 
 

@@ -127,9 +127,11 @@ def test_norm_and_token_shift_sums_a_row_in_one_order(width):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("channels,lens,past,bias", [(40, [1, 2, 3, 300, 1, 4, 205, 6], [0, 1, 2, 0, 9, 0, 4, 0], True), (1048, [513], [0], False), (8, [700, 5], [3, 1], True)])
+@pytest.mark.parametrize("channels,lens,past,bias", [(40, [1, 2, 3, 300, 1, 4, 205, 6], [0, 1, 2, 0, 9, 0, 4, 0], True), (1048, [513], [0], False), (8, [700, 5], [3, 1], True),
+                                                      (24, [1, 2] * 200, [0, 1, 2, 3] * 100, True), (16, [7, 9] * 40, [0, 5] * 40, False)])
 def test_short_convolution_of_many_rows(dtype, channels, lens, past, bias):
-    """Four taps over more rows than 512: runs of four rows that sequences of every length begin and end in."""
+    """Four taps over more rows than 512: runs of four rows that sequences of every length begin and end in, and steps of short
+    sequences, which a thread a channel takes."""
     test_short_convolution_with_carried_inputs(dtype, 4, channels, lens, past, bias)
 
 
