@@ -113,6 +113,21 @@ def test_gemm_f32_sums_in_one_order_whatever_the_kernel(k):
             assert torch.equal(ops.linear(x[:m].contiguous(), off), full[:m]), (n, m, "off")
 
 
+@pytest.mark.parametrize("k", [97, 100])
+def test_gemm_f32_sums_in_one_order_with_many_outputs(k):
+    """So many outputs that the tiles are not shared (at every height) and that few rows take tiles of 32 weight rows, the last ones
+    partial; on and off 16-byte boundaries.  The rows of 300, whose tiles are shared for the last columns alone, give the bits."""
+    n, tail = 25001, 700
+    x, w = rnd((300, k), torch.float32, k), rnd((n, k), torch.float32, 5)
+    off = torch.empty(n * k + 1, dtype=torch.float32, device=w.device)[1:].view(n, k).copy_(w)
+    last = ops.linear(x, w[-tail:].contiguous())
+    full = ops.linear(x, w)
+    assert torch.equal(full[:, -tail:], last)
+    for m in (1, 2, 3, 4, 5, 8, 9, 16, 17, 32, 33, 48, 49, 64, 65, 96, 97, 128, 192):
+        for weight in (w, off):
+            assert torch.equal(ops.linear(x[:m].contiguous(), weight), full[:m]), (m, weight is off)
+
+
 def test_linear_bf16_float32_output():
     x, w = rnd((5, 96), torch.bfloat16, 11), rnd((384, 96), torch.bfloat16, 12)
     assert ops.linear(x, w, out_dtype=torch.float32).dtype is torch.float32
