@@ -348,6 +348,7 @@ cudaError_t launch_tile(float* out, const float* x, const float* w, int M, int N
 
 template <int TM, bool ALIGNED>
 cudaError_t launch_tile_rows(float* out, const float* x, const float* w, int M, int N, int K, cudaStream_t st) {
+    // (the rule's other sides are measured beside launch_rows)
     // Eight blocks a tile where the waves of whole tiles would leave more of the chip idle than the eighths' waves do (clusters
     // of eight reach about seven eighths of the multiprocessors, and their meeting costs about as much again).
     const int per_sm = TM <= 4 ? 2 : 1;
@@ -360,7 +361,14 @@ cudaError_t launch_tile_rows(float* out, const float* x, const float* w, int M, 
 template <bool ALIGNED>
 cudaError_t launch_rows(float* out, const float* x, const float* w, int M, int N, int K, cudaStream_t st) {
     if (M <= FEW_MAX) return launch_few_rows<ALIGNED>(out, x, w, M, N, K, st);
-    // the tile height that pads least; from 97 rows on 128, or 64 where 128 would pad by more than a tenth
+    // The tile height that pads least; from 97 rows on 128, or 64 where 128 would pad by more than a tenth.  Microseconds by height, s: shared
+    // by eight blocks, * what the rules take:
+    //   2,304 outputs of 9,216    17 rows  32 466  32s 106*  48s 124  64s 147      48 rows  32s 159  48s 125*  64s 148     64 rows  48s 186  64s 149*
+    //                             96 rows  32s 216  48s 198*  64s 224  128s 258   128 rows  64s 220  128s 259*  128 1055  192 rows  64s 301*  128s 388
+    //   18,432 outputs of 2,304   17 rows  32 123  32s 126*  48 134  64 175        48 rows  32 213  48 136  48s 149*  64 178
+    //                             96 rows  48 239*  64 314  128 277                128 rows  48 357  64 316  128 279*        192 rows  64 467*  128 551
+    //   256,000 outputs of 2,304  16 rows  the few-row kernel 860*  32 1409        32 rows  32 1424*  32s 1577  48 1601
+    // Narrow outputs of 97 to 128 and 200 to 256 rows would take 64s (85 and 91 % of the time), and 33 to 48 rows of 18,432 whole tiles (91 %).
     if (M <= 32) return launch_tile_rows<2, ALIGNED>(out, x, w, M, N, K, st);
     if (M <= 48 || (M > 64 && M <= 96)) return launch_tile_rows<3, ALIGNED>(out, x, w, M, N, K, st);
     const long long p128 = (M + 127) / 128 * 128LL, p64 = (M + 63) / 64 * 64LL;

@@ -553,6 +553,9 @@ def linear(x, weight: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
     x may be `DeferredRows` (the rows after a deferred norm).  activation: an element-wise form of `UNARY_FORMS`
     on the result (the product's epilogue in the library's own bfloat16 kernels, a kernel of its own elsewhere).
 
+    The weight is a constant: the library's own kernels read it before the kernel ahead of them in the stream has ended.  A
+    weight that a kernel of this library has just written needs another kernel (any of torch's) or an event in between.
+
     float32: the library's own FMA kernel (no tensor cores, no reduced-precision mode).
     bfloat16: up to 16 rows (decode) the weight-streaming tensor-core kernels, from 128 rows the TMA +
     tcgen05 kernels, all with float accumulation and the soft-cap in their epilogue.  17 to 127 rows, and
