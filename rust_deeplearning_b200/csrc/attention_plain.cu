@@ -124,12 +124,14 @@ __global__ void attention_plain_kernel(AttentionArgs a) {
 // ---------------------------------------------------------------------------------------------
 // The same for float rows whose head size is a multiple of four (up to 512): a block of eight warps per (query token, head).
 //
-// What bounds it is the latency of reading a few hundred keys; the one-warp kernel reads a key's row four bytes at a
+// What bounds it is the latency of reading a few dozen to a few hundred keys; the one-warp kernel reads a key's row four bytes at a
 // time in one lane, a chain of head_dim fused multiply-adds behind each load (164 us a layer for 45 queries or 2 single
-// tokens over 40 keys of 256).  Here warp w takes the blocks of 32 absolute positions b with b mod 8 == w: eight lanes share
-// a key (16-byte loads, four keys at a time, sums by exchanges among the eight), the values are read by whole
-// warps, and the warps' sums meet in shared memory in warp order.  The order of operations depends on positions and
-// head size alone, not on the step, so logits stay bit-equal however a request is cut.
+// tokens over 40 keys of 256).  Here the warps take the groups of four absolute positions in turn, so that a short context
+// is short for every warp (with 32 neighbouring positions a warp, 40 keys kept two warps busy for eight passes: 19.9 us a layer,
+// 10.8 now; heads of 32 over up to 60 keys 8.7 and 5.0).  Eight lanes share a key (16-byte loads, four keys at a time, sums by
+// exchanges among the eight), the values are read by whole warps, and the warps' sums meet in shared memory in warp order.
+// The order of operations depends on positions and head size alone, not on the step, so logits stay bit-equal however a
+// request is cut.
 // ---------------------------------------------------------------------------------------------
 constexpr int PF_WARPS = 8;
 
@@ -166,10 +168,13 @@ __global__ void __launch_bounds__(PF_WARPS * 32) attention_f32_kernel(AttentionA
     for (int c = 0; c < VC; ++c) acc[c] = zero4;
     float m = -INFINITY, l = 0.f;
 
-    const int first = lo / 32, b0 = first + ((warp - first) & (PF_WARPS - 1));      // this warp's first block of positions
-    for (int b = b0; b * 32 <= p; b += PF_WARPS) {
-        // lane: where key b * 32 + lane lies (a row of the cache, stored swizzled, or a packed new row)
-        const int j = b * 32 + lane;
+    // Superblock sb: 256 positions; this warp's 32 of them are the groups of four positions 4 (8 g + warp) .. + 3, g = 0..7, lane
+    // 4 g + i holding number i of group g.
+    for (int sb = lo / (32 * PF_WARPS); sb * 32 * PF_WARPS <= p; ++sb) {
+        const int j_warp = sb * 32 * PF_WARPS + 4 * warp;
+        if (j_warp > p) break;                              // no position of this warp's is left
+        // lane: where its key lies (a row of the cache, stored swizzled, or a packed new row)
+        const int j = j_warp + 4 * PF_WARPS * (lane >> 2) + (lane & 3);
         const bool valid = j >= lo && j <= p;
         unsigned long long k_at = 0, v_at = 0;
         int sw = -1;                                        // place of the row in its cache page; -1: a packed new row
@@ -185,10 +190,13 @@ __global__ void __launch_bounds__(PF_WARPS * 32) attention_f32_kernel(AttentionA
                 v_at = (unsigned long long)((const float*)a.v_new + off);
             }
         }
-        // scores: four keys a pass, eight lanes a key
+        // the groups with a visible position
+        const unsigned seen = __ballot_sync(0xffffffffu, valid);
+        const int g0 = seen ? (__ffs(seen) - 1) >> 2 : 8, g1 = seen ? (31 - __clz(seen)) >> 2 : -1;
+        // scores: a group of four keys a pass, eight lanes a key
         float s = 0.f;
 #pragma unroll 2
-        for (int pass = 0; pass < 8; ++pass) {
+        for (int pass = g0; pass <= g1; ++pass) {
             const int key = pass * 4 + (lane >> 3);
             const float4* k4 = reinterpret_cast<const float4*>(__shfl_sync(0xffffffffu, k_at, key));
             const int ksw = __shfl_sync(0xffffffffu, sw, key);
@@ -227,20 +235,24 @@ __global__ void __launch_bounds__(PF_WARPS * 32) attention_f32_kernel(AttentionA
 #pragma unroll
             for (int c = 0; c < VC; ++c) { acc[c].x *= corr; acc[c].y *= corr; acc[c].z *= corr; acc[c].w *= corr; }
         }
-        const int j0 = max(lo - b * 32, 0), j1 = min(p - b * 32, 31);
-#pragma unroll 8
-        for (int jj = j0; jj <= j1; ++jj) {
-            const float pw = __shfl_sync(0xffffffffu, pj, jj);
-            const float4* v4 = reinterpret_cast<const float4*>(__shfl_sync(0xffffffffu, v_at, jj));
-            const int vsw = __shfl_sync(0xffffffffu, sw, jj);
+#pragma unroll 2
+        for (int pass = g0; pass <= g1; ++pass) {
 #pragma unroll
-            for (int c = 0; c < VC; ++c) {
-                const int i = 32 * c + lane;
-                const float4 v = i < chunks ? v4[vsw < 0 ? i : rdl_swizzled_chunk(vsw, i, chunks)] : zero4;
-                acc[c].x = fmaf(pw, v.x, acc[c].x);
-                acc[c].y = fmaf(pw, v.y, acc[c].y);
-                acc[c].z = fmaf(pw, v.z, acc[c].z);
-                acc[c].w = fmaf(pw, v.w, acc[c].w);
+            for (int i4 = 0; i4 < 4; ++i4) {
+                const int key = pass * 4 + i4;
+                const float pw = __shfl_sync(0xffffffffu, pj, key);
+                const float4* v4 = reinterpret_cast<const float4*>(__shfl_sync(0xffffffffu, v_at, key));
+                const int vsw = __shfl_sync(0xffffffffu, sw, key);
+                if (!v4) continue;                          // uniform over the warp: a position that is not seen
+#pragma unroll
+                for (int c = 0; c < VC; ++c) {
+                    const int i = 32 * c + lane;
+                    const float4 v = i < chunks ? v4[vsw < 0 ? i : rdl_swizzled_chunk(vsw, i, chunks)] : zero4;
+                    acc[c].x = fmaf(pw, v.x, acc[c].x);
+                    acc[c].y = fmaf(pw, v.y, acc[c].y);
+                    acc[c].z = fmaf(pw, v.z, acc[c].z);
+                    acc[c].w = fmaf(pw, v.w, acc[c].w);
+                }
             }
         }
     }

@@ -412,6 +412,18 @@ def test_float32_attention_shares_the_keys_among_warps(shape):
     assert_close(got, want, torch.float32, what="float32 attention", f32_tol=c.max_total * 2.0 ** -24)     # sums over the keys
 
 
+@pytest.mark.parametrize("window", [None, 1, 6, 259])
+def test_float32_attention_of_short_and_ragged_contexts(window):
+    """Contexts on both sides of a warp's group of four positions and of the 256 positions eight warps take in turn, windows that
+    begin inside a group; the keys of the cache and a step's own."""
+    c = Case(dtype=torch.float32, seed=34, past=[0, 2, 3, 4, 31, 32, 254, 255, 256, 520], new=[7, 1, 1, 1, 1, 2, 1, 1, 1, 4], n_heads=4,
+             n_kv_heads=2, head_dim=40, page_size=16, window=window)
+    b = c.batch("past")
+    got = ops.attention(c.qkv, b, c.pages, new_kv=c.new_kv(), kind="plain", **c.kw(softcap=5.0))
+    want = ref.attention(c.qkv, b, c.pages, new_kv=c.new_kv(), **c.kw(softcap=5.0))
+    assert_close(got, want, torch.float32, what="float32 attention", f32_tol=c.max_total * 2.0 ** -24)     # sums over the keys
+
+
 @pytest.mark.parametrize("head_dim,n_heads,n_kv_heads,page_size,window,chunk", [
     (256, 8, 4, 64, None, None), (256, 6, 3, 64, 300, None), (80, 8, 2, 48, None, None), (128, 8, 8, 128, None, 150), (64, 8, 1, 64, None, None),
     (32, 8, 4, 16, 200, None), (16, 8, 4, 64, None, None)])
