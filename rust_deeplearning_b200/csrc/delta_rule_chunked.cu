@@ -11,7 +11,7 @@
 // Every P is a product of decays (never a quotient), so nothing overflows however small a decay is.  kd, qd, w, P(0, C), A
 // and B depend on no state: a first launch makes them for all groups of the step at once (a record per group and head, laid
 // out as the second launch reads it), together with beta and v in float.  The second launch walks each sequence's groups:
-// a block of eight warps per 16 columns of a head's state, lane (column, slice) with RPS rows of its column in registers.
+// a block of eight warps per 16 or 32 columns of a head's state, lane (column or two, slice) with RPS rows of its columns in registers.
 // For a group a lane forms its parts of the 16 sums S^T kd_t and S^T qd_t in one pass, the sixteen lanes of a column add
 // them in one round of exchanges, u = T r and o = S^T qd + (B T) r follow as one row of products a lane (the triangular
 // system's inverse T = (I + diag(beta) A)^-1 diag(beta) and B T depend on no state and come with the record), and the
@@ -24,7 +24,7 @@
 namespace {
 
 constexpr int DC_C = 8;             // tokens of a group
-constexpr int DC_COLS = 16;         // columns of a block of the second launch
+constexpr int DC_COLS = 16;         // columns of a block of the second launch, for each column of a lane; a record's v is padded to it
 constexpr int DC_THREADS = 256;
 constexpr int DC_STAGES = 4;
 constexpr int DC_SCALARS = 2 * DC_C * DC_C + DC_C;      // A, B, beta
@@ -34,7 +34,7 @@ constexpr int DC_SCALARS = 2 * DC_C * DC_C + DC_C;      // A, B, beta
 // then T [C][C], B T [C][C], beta [C]; then v [C][columns rounded up to 16].
 template <int RPS> struct DcRecord {
     static constexpr int SLICE = RPS == 4 ? 4 : RPS + 4, VEC = 16 * SLICE, SC = (3 * DC_C + 1) * VEC, V = SC + DC_SCALARS;
-    static constexpr int STAGE = V + DC_C * DC_COLS;          // what a block keeps of a record
+    __host__ __device__ static constexpr int stage(int cols) { return V + DC_C * cols; }      // what a block of so many columns keeps of a record
     __host__ __device__ static int at(int i) { return (i / RPS) * SLICE + (i % RPS); }
     __host__ __device__ static long long floats(int vdim) { return V + (long long)DC_C * ((vdim + DC_COLS - 1) / DC_COLS * DC_COLS); }
 };
@@ -167,14 +167,14 @@ __device__ __forceinline__ void dc_commit() { asm volatile("cp.async.commit_grou
 __device__ __forceinline__ void dc_wait_oldest() { asm volatile("cp.async.wait_group %0;" ::"n"(DC_STAGES - 2) : "memory"); }
 __device__ __forceinline__ void dc_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
-// a record's vectors and scalars, and this block's 16 columns of its v, into a stage
-template <int RPS>
+// a record's vectors and scalars, and this block's COLS columns of its v (those the record has), into a stage
+template <int RPS, int COLS>
 __device__ __forceinline__ void dc_ask(const float* rec, int vp, int c0, float* stage, int tid) {
     using R = DcRecord<RPS>;
     for (int i = 4 * tid; i < R::V; i += 4 * DC_THREADS) dc_copy16(stage + i, rec + i);
-    if (tid < DC_C * DC_COLS / 4) {
-        const int t = tid / (DC_COLS / 4), c = 4 * (tid % (DC_COLS / 4));
-        dc_copy16(stage + R::V + t * DC_COLS + c, rec + R::V + (long long)t * vp + c0 + c);
+    if (tid < DC_C * COLS / 4) {
+        const int t = tid / (COLS / 4), c = 4 * (tid % (COLS / 4));
+        if (c0 + c < vp) dc_copy16(stage + R::V + t * COLS + c, rec + R::V + (long long)t * vp + c0 + c);
     }
 }
 
@@ -203,14 +203,16 @@ __device__ __forceinline__ float dc_sum16(const float (&x)[16], int r) {
     return mine + __shfl_xor_sync(full, send, 1);
 }
 
-template <int RPS>
-__global__ void __launch_bounds__(DC_THREADS) dc_scan_kernel(RecurrenceArgs a, const float* __restrict__ records) {
+// CPL: columns of a lane.
+template <int RPS, int CPL>
+__global__ void __launch_bounds__(DC_THREADS, 2) dc_scan_kernel(RecurrenceArgs a, const float* __restrict__ records) {
     using R = DcRecord<RPS>;
+    constexpr int COLS = DC_COLS * CPL, STAGE = R::stage(COLS);
     extern __shared__ __align__(16) float dc_ring[];
     rdl_grid_wait();
     rdl_grid_launch_dependents();
     const int dim = a.dim, vdim = a.vdim;
-    const int seq = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * DC_COLS;
+    const int seq = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * COLS;
     const int row0 = a.seq_start[seq], n = a.seq_start[seq + 1] - row0;
     if (n <= 0) return;
     if (a.tok_pos[row0] < 0) return;          // a padding sequence of a fixed-size batch
@@ -221,8 +223,7 @@ __global__ void __launch_bounds__(DC_THREADS) dc_scan_kernel(RecurrenceArgs a, c
     }
     const int groups = (n + DC_C - 1) / DC_C;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int c = lane >> 4, r = lane & 15, bc = 2 * warp + c, col = c0 + bc;
-    const bool col_ok = col < vdim;
+    const int c = lane >> 4, r = lane & 15, bc = (2 * warp + c) * CPL, col = c0 + bc;      // this lane's columns: col .. col + CPL - 1
     const unsigned full = 0xffffffffu;
     const int vp = (vdim + DC_COLS - 1) / DC_COLS * DC_COLS;
     const long long rec_floats = R::floats(vdim);
@@ -230,84 +231,114 @@ __global__ void __launch_bounds__(DC_THREADS) dc_scan_kernel(RecurrenceArgs a, c
     const long long rec_step = (long long)a.n_heads * rec_floats;
 #pragma unroll
     for (int d = 0; d < DC_STAGES - 1; ++d) {
-        if (d < groups) dc_ask<RPS>(rec0 + d * rec_step, vp, c0, dc_ring + d * R::STAGE, tid);
+        if (d < groups) dc_ask<RPS, COLS>(rec0 + d * rec_step, vp, c0, dc_ring + d * STAGE, tid);
         dc_commit();
     }
     float* S = a.state + (((long long)a.slots[seq] * a.n_heads + h) * dim) * vdim + col;
-    float s[RPS];
+    float s[CPL][RPS];
 #pragma unroll
-    for (int i = 0; i < RPS; ++i) s[i] = (col_ok && r * RPS + i < dim) ? S[(long long)(r * RPS + i) * vdim] : 0.f;
+    for (int q = 0; q < CPL; ++q)
+#pragma unroll
+        for (int i = 0; i < RPS; ++i) s[q][i] = (col + q < vdim && r * RPS + i < dim) ? S[(long long)(r * RPS + i) * vdim + q] : 0.f;
     float* out = a.out + (long long)row0 * a.n_heads * vdim + (long long)h * vdim + col;
     const int out_step = a.n_heads * vdim;
 
     for (int gi = 0; gi < groups; ++gi) {
-        const float* stage = dc_ring + (gi % DC_STAGES) * R::STAGE;
+        const float* stage = dc_ring + (gi % DC_STAGES) * STAGE;
         dc_wait_oldest();
         __syncthreads();            // this group's record is there for every warp, and every warp is done with the one before
         const int ahead = gi + DC_STAGES - 1;
-        if (ahead < groups) dc_ask<RPS>(rec0 + ahead * rec_step, vp, c0, dc_ring + (ahead % DC_STAGES) * R::STAGE, tid);
+        if (ahead < groups) dc_ask<RPS, COLS>(rec0 + ahead * rec_step, vp, c0, dc_ring + (ahead % DC_STAGES) * STAGE, tid);
         dc_commit();
         const float* mine = stage + r * R::SLICE;
         // this lane's parts of S^T kd_t (x[t]) and S^T qd_t (x[C + t])
-        float x[2 * DC_C];
+        float x[CPL][2 * DC_C];
 #pragma unroll
         for (int t = 0; t < 2 * DC_C; ++t) {
-            float acc0 = 0.f, acc1 = 0.f;
+            float acc0[CPL], acc1[CPL];
+#pragma unroll
+            for (int q = 0; q < CPL; ++q) acc0[q] = acc1[q] = 0.f;
 #pragma unroll
             for (int i = 0; i < RPS; i += 4) {
                 const float4 m = *reinterpret_cast<const float4*>(mine + t * R::VEC + i);
-                acc0 = fmaf(s[i], m.x, acc0); acc1 = fmaf(s[i + 1], m.y, acc1); acc0 = fmaf(s[i + 2], m.z, acc0); acc1 = fmaf(s[i + 3], m.w, acc1);
+#pragma unroll
+                for (int q = 0; q < CPL; ++q) {
+                    acc0[q] = fmaf(s[q][i], m.x, acc0[q]); acc1[q] = fmaf(s[q][i + 1], m.y, acc1[q]);
+                    acc0[q] = fmaf(s[q][i + 2], m.z, acc0[q]); acc1[q] = fmaf(s[q][i + 3], m.w, acc1[q]);
+                }
             }
-            x[t] = acc0 + acc1;
+#pragma unroll
+            for (int q = 0; q < CPL; ++q) x[q][t] = acc0[q] + acc1[q];
         }
-        const float z = dc_sum16(x, r);
         const float* sc = stage + R::SC;
         // Lanes 0..7 of a column hold S^T kd_t, lanes 8..15 S^T qd_t.  r_t = v_t - S^T kd_t goes to every lane; lane t then
         // forms u_t = (T r)_t and lane 8 + t o_t = S^T qd_t + (B T r)_t, a row of eight products each.
         const int left = n - gi * DC_C;
         const int tt = r & 7;
-        const float val = r < DC_C ? stage[R::V + tt * DC_COLS + bc] - z : z;
-        float rj[DC_C];
-#pragma unroll
-        for (int j = 0; j < DC_C; ++j) rj[j] = __shfl_sync(full, val, j, 16);
         const float* mrow = sc + r * DC_C;            // row t of T for lanes 0..7, row t of B T for lanes 8..15
         const float4 m_lo = *reinterpret_cast<const float4*>(mrow), m_hi = *reinterpret_cast<const float4*>(mrow + 4);
-        float acc = r < DC_C ? 0.f : z;
-        acc = fmaf(m_lo.x, rj[0], acc); acc = fmaf(m_lo.y, rj[1], acc); acc = fmaf(m_lo.z, rj[2], acc); acc = fmaf(m_lo.w, rj[3], acc);
-        acc = fmaf(m_hi.x, rj[4], acc); acc = fmaf(m_hi.y, rj[5], acc); acc = fmaf(m_hi.z, rj[6], acc); acc = fmaf(m_hi.w, rj[7], acc);
-        if (r >= DC_C && col_ok && tt < left) out[(long long)(gi * DC_C + tt) * out_step] = acc;
-        float u[DC_C];
+        float u[CPL][DC_C];
 #pragma unroll
-        for (int j = 0; j < DC_C; ++j) u[j] = __shfl_sync(full, acc, j, 16);
+        for (int q = 0; q < CPL; ++q) {
+            const float z = dc_sum16(x[q], r);
+            const float val = r < DC_C ? stage[R::V + tt * COLS + bc + q] - z : z;
+            float rj[DC_C];
+#pragma unroll
+            for (int j = 0; j < DC_C; ++j) rj[j] = __shfl_sync(full, val, j, 16);
+            float acc = r < DC_C ? 0.f : z;
+            acc = fmaf(m_lo.x, rj[0], acc); acc = fmaf(m_lo.y, rj[1], acc); acc = fmaf(m_lo.z, rj[2], acc); acc = fmaf(m_lo.w, rj[3], acc);
+            acc = fmaf(m_hi.x, rj[4], acc); acc = fmaf(m_hi.y, rj[5], acc); acc = fmaf(m_hi.z, rj[6], acc); acc = fmaf(m_hi.w, rj[7], acc);
+            if (r >= DC_C && col + q < vdim && tt < left) out[(long long)(gi * DC_C + tt) * out_step + q] = acc;
+#pragma unroll
+            for (int j = 0; j < DC_C; ++j) u[q][j] = __shfl_sync(full, acc, j, 16);
+        }
         // S' = P(0, C) (.) S + sum_j w_j u_j^T
 #pragma unroll
         for (int i = 0; i < RPS; i += 4) {
             const float4 pc = *reinterpret_cast<const float4*>(mine + 3 * DC_C * R::VEC + i);
-            s[i] *= pc.x; s[i + 1] *= pc.y; s[i + 2] *= pc.z; s[i + 3] *= pc.w;
+#pragma unroll
+            for (int q = 0; q < CPL; ++q) { s[q][i] *= pc.x; s[q][i + 1] *= pc.y; s[q][i + 2] *= pc.z; s[q][i + 3] *= pc.w; }
         }
 #pragma unroll
         for (int j = 0; j < DC_C; ++j) {
 #pragma unroll
             for (int i = 0; i < RPS; i += 4) {
                 const float4 w4 = *reinterpret_cast<const float4*>(mine + (2 * DC_C + j) * R::VEC + i);
-                s[i] = fmaf(w4.x, u[j], s[i]); s[i + 1] = fmaf(w4.y, u[j], s[i + 1]); s[i + 2] = fmaf(w4.z, u[j], s[i + 2]); s[i + 3] = fmaf(w4.w, u[j], s[i + 3]);
+#pragma unroll
+                for (int q = 0; q < CPL; ++q) {
+                    s[q][i] = fmaf(w4.x, u[q][j], s[q][i]); s[q][i + 1] = fmaf(w4.y, u[q][j], s[q][i + 1]);
+                    s[q][i + 2] = fmaf(w4.z, u[q][j], s[q][i + 2]); s[q][i + 3] = fmaf(w4.w, u[q][j], s[q][i + 3]);
+                }
             }
         }
     }
     dc_wait_all();
 #pragma unroll
-    for (int i = 0; i < RPS; ++i)
-        if (col_ok && r * RPS + i < dim) S[(long long)(r * RPS + i) * vdim] = s[i];
+    for (int q = 0; q < CPL; ++q)
+#pragma unroll
+        for (int i = 0; i < RPS; ++i)
+            if (col + q < vdim && r * RPS + i < dim) S[(long long)(r * RPS + i) * vdim + q] = s[q][i];
+}
+
+template <int RPS, int CPL>
+cudaError_t dc_launch_scan(const RecurrenceArgs* a, const float* records, cudaStream_t st) {
+    constexpr int COLS = DC_COLS * CPL;
+    const size_t smem = (size_t)DC_STAGES * DcRecord<RPS>::stage(COLS) * sizeof(float);
+    const cudaError_t e = rdl_allow_shared<dc_scan_kernel<RPS, CPL>>((int)smem);
+    if (e != cudaSuccess) return e;
+    return rdl_launch(dc_scan_kernel<RPS, CPL>, dim3(a->n_seqs, a->n_heads, (a->vdim + COLS - 1) / COLS), dim3(DC_THREADS), smem, st, *a, records);
 }
 
 template <typename T, int RPS>
 int dc_launch(const RecurrenceArgs* a, float* records, int max_groups, cudaStream_t st) {
-    using R = DcRecord<RPS>;
-    const size_t smem = (size_t)DC_STAGES * R::STAGE * sizeof(float);
-    RDL_CUDA((rdl_allow_shared<dc_scan_kernel<RPS>>(smem)), "delta_rule_chunked");
     RDL_CHECK_EX(rdl_launch(dc_record_kernel<T, RPS>, dim3(max_groups, a->n_heads), dim3(128), 0, st, *a, records), "delta_rule_chunked (records)");
-    RDL_CHECK_EX(rdl_launch(dc_scan_kernel<RPS>, dim3(a->n_seqs, a->n_heads, (a->vdim + DC_COLS - 1) / DC_COLS), dim3(DC_THREADS), smem, st, *a,
-                            (const float*)records), "delta_rule_chunked (scan)");
+    const char* ev = getenv("RDL_X_CPL");
+    // Two columns a lane halve the reads of a group's vectors from shared memory, which bound the walk where blocks share a
+    // multiprocessor; with one block each the walk is bound by its own chain, which two columns lengthen.  Two blocks of one
+    // column fit a multiprocessor.  Both launches, 16 heads of 128 x 128, one column against two: 1 x 1,500 tokens 506 / 610 us, 2 x 700
+    // (256 blocks) 262 / 305, 4 x 400 (512) 299 / 203, 16 x 100 303 / 211, 64 x 60 850 / 596, 200 + 633 + 1,066 + 1,500 810 / 634.
+    const bool two = (long long)a->n_seqs * a->n_heads * ((a->vdim + DC_COLS - 1) / DC_COLS) > 2 * rdl_sm_count();
+    RDL_CHECK_EX((two ? dc_launch_scan<RPS, 2>(a, records, st) : dc_launch_scan<RPS, 1>(a, records, st)), "delta_rule_chunked (scan)");
     return 0;
 }
 

@@ -282,6 +282,28 @@ def test_state_space_in_chunks(sizes):
         ops.state_space_scan(rows[:, 4:], dt_rows, state=st, n_seqs=r.n, kind="chunked", **r.where(), **{**kw, "b_col": kw["b_col"] - 4, "c_col": kw["c_col"] - 4})
 
 
+@pytest.mark.parametrize("d,e", [(20, 33), (64, 40), (128, 48), (128, 64)])      # columns that end inside a lane's pair, a warp's and a block's
+def test_delta_rule_two_columns_a_lane(d, e):
+    """So many sequences that a lane takes two columns: the bits of every sequence as a step of its own (one column a lane)."""
+    H, lens = 2, [9, 1, 16, 23, 8] * 24
+    r = Rows(lens, [0] * len(lens))
+    rows = rnd((r.T, H * e), torch.bfloat16, 60, 0.8)
+    q_f, k_f, g_f = rnd((r.T, H * d), torch.float32, 61, 0.1), rnd((r.T, H * d), torch.float32, 62, 0.1), torch.sigmoid(rnd((r.T, H * d), torch.float32, 63, 2.0))
+    beta_f = torch.sigmoid(rnd((r.T, H), torch.float32, 64, 1.0))
+    state = rnd((r.n_slots, H, d, e), torch.float32, 65, 0.5)
+    kw = dict(v_col=0, n_heads=H, n_key_heads=H, dim=d, vdim=e, kind="chunked")
+    assert r.n * H * -(-e // 16) > 2 * ops.sm_count(0)
+    st = state.clone()
+    got = ops.delta_rule_scan(rows, q_f=q_f, k_f=k_f, g_f=g_f, beta_f=beta_f, state=st, n_seqs=r.n, **r.where(), **kw)
+    for s in range(10):
+        sl = slice(int(r.starts[s]), int(r.starts[s + 1]))
+        o = Rows([lens[s]], [0])
+        o.slots = r.slots[s:s + 1].contiguous()
+        alone = ops.delta_rule_scan(rows[sl], q_f=q_f[sl], k_f=k_f[sl], g_f=g_f[sl], beta_f=beta_f[sl], state=state, n_seqs=1, **o.where(), **kw)
+        assert torch.equal(alone, got[sl])
+        assert torch.equal(state[int(r.slot_ids[s])], st[int(r.slot_ids[s])])
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("sizes", [dict(H=4, J=2, d=16, e=24, lens=[33, 1, 2], past=[0, 7, 0]), dict(H=3, J=1, d=12, e=20, lens=[5, 70], past=[3, 0]),
                                    dict(H=2, J=2, d=64, e=64, lens=[40], past=[0]), dict(H=1, J=1, d=130, e=33, lens=[6, 1], past=[2, 0]),
