@@ -15,10 +15,12 @@
 //     different banks); the eight warps of a block are the eight runs, whose sums meet in shared memory once a tile.
 //     Blocks are persistent and the ring runs on from tile to tile; weights are asked for before the wait on the
 //     kernel before.
-//   * Above, the float units bound it.  A block forms a tile of 32, 48, 64 or 128 rows by 128 columns, a thread 2 to 8 by 8
+//   * Above, the float units bound it.  A block forms a tile of 32, 48, 64 or 128 rows by 128 columns, a thread 4 to 8 by 8
 //     of them, both operands' rows in shared memory as they lie in memory (no transposition: the two-wide instruction
 //     takes neighbouring k).  Where the tiles alone do not fill the chip, eight blocks (a cluster) share a tile, a run of k
 //     each, and add up through distributed shared memory.
+//     A thread's 6 or 8 by 8 sums cost 14 or 16 reads of 16 bytes for 96 or 128 two-wide multiply-adds; with 3 by 8 (11 for 48) the
+//     reads from shared memory were the bound: 2,304 outputs of 9,216 for 48 rows 125 -> 110 us, 18,432 of 2,304 146 -> 122 (33 TFLOP/s).
 // Both take operands that are not 16-byte aligned (or K not a multiple of four) by 4-byte copies.
 // (The reference's product is an f32 library GEMM: rustml/core/main/src/core/tensor/ops.rs:806-823;
 // y = x W^T with W [out, in]: rustml/nn/main/src/core/linear.rs:12-15, :168-169.)
@@ -189,8 +191,8 @@ cudaError_t launch_few_rows(float* out, const float* x, const float* w, int M, i
 // ---- many rows ----
 
 constexpr int TN = 8, BN = 16 * TN;
-// Two blocks a multiprocessor up to 64 rows a tile (hence the shorter ring there), one with 128.
-__host__ __device__ constexpr int tile_stages(int tm) { return tm == 4 ? 2 : 3; }
+// Blocks a multiprocessor: what the registers of 16 TY threads with 8 TM sums each allow.
+__host__ __device__ constexpr int tile_blocks(int tm, int ty) { return ty == 8 ? (tm <= 6 ? 3 : 2) : (tm <= 4 ? 2 : 1); }
 
 __device__ __forceinline__ uint32_t f32_cluster_rank() {
     uint32_t r;
@@ -208,12 +210,13 @@ __device__ __forceinline__ float f32_ld_remote(uint32_t addr, uint32_t rank) {
     return v;
 }
 
-// A tile of 16 TM rows by 128 columns; thread (ty, tx) has rows ty + 16 i and columns tx + 16 j.  SHARED: the block is one of a
+// A tile of TY TM rows by 128 columns; thread (ty, tx) has rows ty + TY i and columns tx + 16 j.  SHARED: the block is one of a
 // cluster of eight along z, each with a run of k.
-template <int TM, bool SHARED, bool ALIGNED>
-__global__ void __launch_bounds__(256, TM <= 4 ? 2 : 1) gemm_f32_tile_kernel(float* __restrict__ out, const float* __restrict__ x,
+template <int TM, int TY, int TILE_STAGES, bool SHARED, bool ALIGNED>
+__global__ void __launch_bounds__(16 * TY, tile_blocks(TM, TY)) gemm_f32_tile_kernel(float* __restrict__ out, const float* __restrict__ x,
                                                                             const float* __restrict__ w, int M, int N, int K) {
-    constexpr int BM = 16 * TM, STAGE = (BM + BN) * PITCH, TILE_STAGES = tile_stages(TM);       // STAGE: floats
+    constexpr int BM = TY * TM, STAGE = (BM + BN) * PITCH, RP = 2 * TY;      // RP: rows a pass of copies takes
+           // STAGE: floats
     extern __shared__ __align__(16) float sm[];
     float* sums = sm + TILE_STAGES * STAGE;                       // [BM][BN]: the runs' sums so far (SHARED: this block's run)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -226,16 +229,16 @@ __global__ void __launch_bounds__(256, TM <= 4 ? 2 : 1) gemm_f32_tile_kernel(flo
     auto copy = [&](int k, int k_hi, int s, bool weights) {      // the chunk from k on into stage s
         if (weights) {
 #pragma unroll
-            for (int i = 0; i < BN / 32; ++i) {
-                const int r = i * 32 + (tid >> 3), kk = k + (tid & 7) * 4, n = n0 + r;
+            for (int i = 0; i < BN / RP; ++i) {
+                const int r = i * RP + (tid >> 3), kk = k + (tid & 7) * 4, n = n0 + r;
                 const bool ok = n < N && kk < k_hi;
                 copy4<ALIGNED>(base + (uint32_t)((s * STAGE + (BM + r) * PITCH + (tid & 7) * 4) * 4), ok ? w + (long long)n * K + kk : w, ok ? k_hi - kk : 0);
             }
         } else {
 #pragma unroll
-            for (int i = 0; i < (BM + 31) / 32; ++i) {
-                const int r = i * 32 + (tid >> 3), kk = k + (tid & 7) * 4, m = m0 + r;
-                if (BM % 32 && r >= BM) continue;
+            for (int i = 0; i < (BM + RP - 1) / RP; ++i) {
+                const int r = i * RP + (tid >> 3), kk = k + (tid & 7) * 4, m = m0 + r;
+                if (BM % RP && r >= BM) continue;
                 const bool ok = m < M && kk < k_hi;
                 copy4<ALIGNED>(base + (uint32_t)((s * STAGE + r * PITCH + (tid & 7) * 4) * 4), ok ? x + (long long)m * K + kk : x, ok ? k_hi - kk : 0);
             }
@@ -277,7 +280,7 @@ __global__ void __launch_bounds__(256, TM <= 4 ? 2 : 1) gemm_f32_tile_kernel(flo
                 for (int j = 0; j < TN; ++j) b[j] = lds_pairs(wa + (j * 16 * PITCH + q * 4) * 4);
 #pragma unroll
                 for (int i = 0; i < TM; ++i) {
-                    const Pairs a = lds_pairs(xa + (i * 16 * PITCH + q * 4) * 4);
+                    const Pairs a = lds_pairs(xa + (i * TY * PITCH + q * 4) * 4);
 #pragma unroll
                     for (int j = 0; j < TN; ++j) {
                         acc[i][j] = ffma2(a.lo, b[j].lo, acc[i][j]);
@@ -290,7 +293,7 @@ __global__ void __launch_bounds__(256, TM <= 4 ? 2 : 1) gemm_f32_tile_kernel(flo
         const bool first = SHARED || g == 0, last = !SHARED && g == RUNS - 1;
 #pragma unroll
         for (int i = 0; i < TM; ++i) {
-            const int r = ty + 16 * i;
+            const int r = ty + TY * i;
 #pragma unroll
             for (int j = 0; j < TN; ++j) {
                 const int c = tx + 16 * j;
@@ -306,7 +309,7 @@ __global__ void __launch_bounds__(256, TM <= 4 ? 2 : 1) gemm_f32_tile_kernel(flo
         const uint32_t rank = f32_cluster_rank();
         const uint32_t sums_s = base + (uint32_t)(TILE_STAGES * STAGE * 4);
         constexpr int ROWS_EACH = BM / RUNS;
-        for (int i = tid; i < ROWS_EACH * BN; i += 256) {
+        for (int i = tid; i < ROWS_EACH * BN; i += 16 * TY) {
             const int r = (int)rank * ROWS_EACH + i / BN, c = i % BN;
             float v[RUNS];
 #pragma unroll
@@ -319,15 +322,15 @@ __global__ void __launch_bounds__(256, TM <= 4 ? 2 : 1) gemm_f32_tile_kernel(flo
     }
 }
 
-template <int TM, bool SHARED, bool ALIGNED>
+template <int TM, int TY, int STAGES, bool SHARED, bool ALIGNED>
 cudaError_t launch_tile(float* out, const float* x, const float* w, int M, int N, int K, cudaStream_t st) {
-    constexpr int BM = 16 * TM;
-    constexpr size_t smem = (size_t)(tile_stages(TM) * (BM + BN) * PITCH + BM * BN) * 4;
-    const cudaError_t e = rdl_allow_shared<gemm_f32_tile_kernel<TM, SHARED, ALIGNED>>((int)smem);
+    constexpr int BM = TY * TM;
+    constexpr size_t smem = (size_t)(STAGES * (BM + BN) * PITCH + BM * BN) * 4;
+    const cudaError_t e = rdl_allow_shared<gemm_f32_tile_kernel<TM, TY, STAGES, SHARED, ALIGNED>>((int)smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((N + BN - 1) / BN, (M + BM - 1) / BM, SHARED ? RUNS : 1);
-    cfg.blockDim = dim3(256);
+    cfg.blockDim = dim3(16 * TY);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
@@ -343,36 +346,49 @@ cudaError_t launch_tile(float* out, const float* x, const float* w, int M, int N
     }
     cfg.attrs = attr;
     cfg.numAttrs = n;
-    return cudaLaunchKernelEx(&cfg, gemm_f32_tile_kernel<TM, SHARED, ALIGNED>, out, x, w, M, N, K);
+    return cudaLaunchKernelEx(&cfg, gemm_f32_tile_kernel<TM, TY, STAGES, SHARED, ALIGNED>, out, x, w, M, N, K);
 }
 
-template <int TM, bool ALIGNED>
+template <int TM, int TY, bool ALIGNED>
 cudaError_t launch_tile_rows(float* out, const float* x, const float* w, int M, int N, int K, cudaStream_t st) {
     // (the rule's other sides are measured beside launch_rows)
     // Eight blocks a tile where the waves of whole tiles would leave more of the chip idle than the eighths' waves do (clusters
     // of eight reach about seven eighths of the multiprocessors, and their meeting costs about as much again).
-    const int per_sm = TM <= 4 ? 2 : 1;
-    const long long tiles = (long long)((N + BN - 1) / BN) * ((M + 16 * TM - 1) / (16 * TM));
-    const long long slots = (long long)rdl_sm_count() * per_sm, slots8 = slots * 7 / 8;
-    const double whole = (double)((tiles + slots - 1) / slots), eighths = (double)((tiles * RUNS + slots8 - 1) / slots8) / RUNS * 1.15;
-    return whole <= eighths ? launch_tile<TM, false, ALIGNED>(out, x, w, M, N, K, st) : launch_tile<TM, true, ALIGNED>(out, x, w, M, N, K, st);
+    constexpr int WHOLE = TY == 16 ? 3 : 2;                       // chunks of the ring with as many blocks as a multiprocessor takes
+    const long long tiles = (long long)((N + BN - 1) / BN) * ((M + TY * TM - 1) / (TY * TM)), blocks8 = tiles * RUNS;
+    const long long sms8 = rdl_sm_count() * 7LL / 8, slots = (long long)rdl_sm_count() * tile_blocks(TM, TY), slots8 = sms8 * tile_blocks(TM, TY);
+    const double whole = (double)((tiles + slots - 1) / slots), eighths = (double)((blocks8 + slots8 - 1) / slots8) / RUNS * 1.15;
+    if (whole <= eighths) return launch_tile<TM, TY, WHOLE, false, ALIGNED>(out, x, w, M, N, K, st);
+    // A shared tile's run of k is a few chunks long, and fewer blocks on a multiprocessor hide less of the wait for them: a deeper
+    // ring where the clusters leave room for it (4,096 outputs of 2,304, 48 rows, 256 blocks: 42 us with two chunks, 33 with three.
+    // Where it takes a multiprocessor from a cluster it costs a second wave: 2,304 of 9,216, 144 blocks, 110 and, five chunks, 142).
+    if constexpr (TY == 8) {
+        if (blocks8 <= sms8) return launch_tile<TM, TY, 5, true, ALIGNED>(out, x, w, M, N, K, st);
+        if constexpr (TM <= 6) {
+            if (4 * blocks8 > 5 * sms8 && blocks8 <= 2 * sms8) return launch_tile<TM, TY, 3, true, ALIGNED>(out, x, w, M, N, K, st);
+        }
+    }
+    return launch_tile<TM, TY, WHOLE, true, ALIGNED>(out, x, w, M, N, K, st);
 }
 
 template <bool ALIGNED>
 cudaError_t launch_rows(float* out, const float* x, const float* w, int M, int N, int K, cudaStream_t st) {
     if (M <= FEW_MAX) return launch_few_rows<ALIGNED>(out, x, w, M, N, K, st);
-    // The tile height that pads least; from 97 rows on 128, or 64 where 128 would pad by more than a tenth.  Microseconds by height, s: shared
-    // by eight blocks, * what the rules take:
-    //   2,304 outputs of 9,216    17 rows  32 466  32s 106*  48s 124  64s 147      48 rows  32s 159  48s 125*  64s 148     64 rows  48s 186  64s 149*
-    //                             96 rows  32s 216  48s 198*  64s 224  128s 258   128 rows  64s 220  128s 259*  128 1055  192 rows  64s 301*  128s 388
-    //   18,432 outputs of 2,304   17 rows  32 123  32s 126*  48 134  64 175        48 rows  32 213  48 136  48s 149*  64 178
-    //                             96 rows  48 239*  64 314  128 277                128 rows  48 357  64 316  128 279*        192 rows  64 467*  128 551
-    //   256,000 outputs of 2,304  16 rows  the few-row kernel 860*  32 1409        32 rows  32 1424*  32s 1577  48 1601
-    // Narrow outputs of 97 to 128 and 200 to 256 rows would take 64s (85 and 91 % of the time), and 33 to 48 rows of 18,432 whole tiles (91 %).
-    if (M <= 32) return launch_tile_rows<2, ALIGNED>(out, x, w, M, N, K, st);
-    if (M <= 48 || (M > 64 && M <= 96)) return launch_tile_rows<3, ALIGNED>(out, x, w, M, N, K, st);
-    const long long p128 = (M + 127) / 128 * 128LL, p64 = (M + 63) / 64 * 64LL;
-    return 10 * p128 > 11 * p64 ? launch_tile_rows<4, ALIGNED>(out, x, w, M, N, K, st) : launch_tile_rows<8, ALIGNED>(out, x, w, M, N, K, st);
+    // The tile height that pads least; from 97 rows on 128 where such tiles give nine tenths of the multiprocessors one and 128 pads by
+    // at most a tenth more than 64, else 64.  Microseconds by height, s: shared by eight blocks, * what the rules take; in brackets what
+    // tiles of half as many sums a thread (16 threads along the rows) took:
+    //   2,304 outputs of 9,216    32 rows  32s 84* (106)   48 rows  32s 115  48s 110* (125)  64s 140     64 rows  32s 115  48s 156  64s 140* (149)
+    //                             90 rows  32s 155  48s 156* (188)  64s 205    120 rows  32s 198  48s 204  64s 208* (258)  128s 258
+    //                            200 rows  32s 301  48s 308  64s 331* (387)  128s 387   256 rows  48s 348  64s 330* (388)  128s 388
+    //   18,432 outputs of 2,304   32 rows  32 109  32s 93* (125)   48 rows  32s 172  48 143  48s 122* (146)  64s 165     64 rows  64 173  64s 165* (172)
+    //                             90 rows  48s 227* (238)  64 294  128 275     120 rows  64 295  64s 314  128 278* (278)    200 rows  48s 539  128 550* (550)
+    //   4,096 outputs of 2,304    32 rows  32s 25* (31)   48 rows  48s 33* (35)   64 rows  32s 52  64s 40* (41)   90 rows  48s 67* (70)  120 rows  64s 78* (109)
+    //   256,000 outputs of 2,304  45 rows  48 1484* (1605)
+    if (M <= 32) return launch_tile_rows<4, 8, ALIGNED>(out, x, w, M, N, K, st);
+    if (M <= 48 || (M > 64 && M <= 96)) return launch_tile_rows<6, 8, ALIGNED>(out, x, w, M, N, K, st);
+    const long long p128 = (M + 127) / 128 * 128LL, p64 = (M + 63) / 64 * 64LL, tiles128 = (N + BN - 1) / BN * (p128 / 128);
+    return 10 * tiles128 < 9LL * rdl_sm_count() || 10 * p128 > 11 * p64 ? launch_tile_rows<8, 8, ALIGNED>(out, x, w, M, N, K, st)
+                                                                        : launch_tile_rows<8, 16, ALIGNED>(out, x, w, M, N, K, st);
 }
 
 }  // namespace

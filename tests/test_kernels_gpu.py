@@ -128,6 +128,19 @@ def test_gemm_f32_sums_in_one_order_with_many_outputs(k):
             assert torch.equal(ops.linear(x[:m].contiguous(), weight), full[:m]), (m, weight is off)
 
 
+@pytest.mark.parametrize("n", [1000, 4000, 5000, 60001])      # shared tiles with rings of five, three and two chunks; whole tiles
+def test_gemm_f32_sums_in_one_order_at_every_ring_depth(n):
+    """k of 300: runs of 40, the last one shorter, chunks that end early; rows on both sides of every tile height."""
+    k, tail = 300, 130
+    x, w = rnd((130, k), torch.float32, 3), rnd((n, k), torch.float32, n)
+    off = torch.empty(n * k + 1, dtype=torch.float32, device=w.device)[1:].view(n, k).copy_(w)
+    rows = ops.linear(x, w)
+    assert torch.equal(rows[:, -tail:], torch.cat([ops.linear(x[i:i + 10].contiguous(), w[-tail:].contiguous()) for i in range(0, 130, 10)]))
+    for m in (17, 32, 33, 48, 49, 64, 65, 96, 97, 128):
+        for weight in (w, off):
+            assert torch.equal(ops.linear(x[:m].contiguous(), weight), rows[:m]), (m, weight is off)
+
+
 def test_linear_bf16_float32_output():
     x, w = rnd((5, 96), torch.bfloat16, 11), rnd((384, 96), torch.bfloat16, 12)
     assert ops.linear(x, w, out_dtype=torch.float32).dtype is torch.float32
