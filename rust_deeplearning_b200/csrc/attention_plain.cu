@@ -127,17 +127,23 @@ __global__ void attention_plain_kernel(AttentionArgs a) {
 // What bounds it is the latency of reading a few dozen to a few hundred keys; the one-warp kernel reads a key's row four bytes at a
 // time in one lane, a chain of head_dim fused multiply-adds behind each load (164 us a layer for 45 queries or 2 single
 // tokens over 40 keys of 256).  Here the warps take the groups of four absolute positions in turn, so that a short context
-// is short for every warp (with 32 neighbouring positions a warp, 40 keys kept two warps busy for eight passes: 19.9 us a layer,
-// 10.8 now; heads of 32 over up to 60 keys 8.7 and 5.0).  Eight lanes share a key (16-byte loads, four keys at a time, sums by
-// exchanges among the eight), the values are read by whole warps, and the warps' sums meet in shared memory in warp order.
-// The order of operations depends on positions and head size alone, not on the step, so logits stay bit-equal however a
-// request is cut.
+// is short for every warp.  Eight lanes share a key (16-byte loads, four keys at a time, sums by exchanges among the eight), the
+// values are read by whole warps, and the warps' sums meet in shared memory in warp order.  The order of operations depends on
+// positions and head size alone, not on the step, so logits stay bit-equal however a request is cut.
+// What keeps it fast behind long contexts is the number of loads in flight: where all 32 of a warp's positions are visible the
+// loops have fixed lengths, elsewhere what is left over does not come one by one, and the registers leave room for four blocks a
+// multiprocessor (heads of up to 64; three up to 128).  A test of every position's address between the loads instead kept the
+// next load behind the test.  One token, microseconds with 32 neighbouring positions a warp / with that test / now:
+//     heads of 256:  40 keys 10.2 / 6.6 / 5.5    250 11.0 / 15.9 / 11.8    500 19.0 / 29.0 / 18.1    1,000 35.6 / 54.8 / 32.7    8,000 310 / 476 / 280
+//     heads of 128:  40 keys 10.7 / 6.4 / 4.8    250 11.0 / 15.5 /  8.6    500 19.5 / 28.4 / 13.8    1,000 36.4 / 54.3 / 25.0    8,000 290 / 445 / 190
+// and a prompt of 1,500 tokens 1,399 / 1,823 / 1,245 (8 heads of 256), 407 / 424 / 368 (6 of 32).  Contexts of 210 to 255 keys
+// of 256 are what neighbouring positions still do better (by 3 to 8 %: there the last places come in fewer trips).
 // ---------------------------------------------------------------------------------------------
 constexpr int PF_WARPS = 8;
 
-// NC: 32-value slices of a head (head_dim <= 32 NC).
+// NC: 32-value slices of a head (head_dim <= 32 NC).  Wider heads are left to the compiler (bounds of one block: 0.6 of the speed).
 template <int NC>
-__global__ void __launch_bounds__(PF_WARPS * 32) attention_f32_kernel(AttentionArgs a) {
+__global__ void __launch_bounds__(PF_WARPS * 32, NC <= 2 ? 4 : NC == 4 ? 3 : 0) attention_f32_kernel(AttentionArgs a) {
     constexpr int VC = (NC + 3) / 4;                       // 128-value slices of a head
     __shared__ float4 part[PF_WARPS][VC][32];
     __shared__ float part_m[PF_WARPS], part_l[PF_WARPS];
@@ -190,13 +196,13 @@ __global__ void __launch_bounds__(PF_WARPS * 32) attention_f32_kernel(AttentionA
                 v_at = (unsigned long long)((const float*)a.v_new + off);
             }
         }
-        // the groups with a visible position
+        // the groups with a visible position, and its places: neighbours, since positions rise with the lane
         const unsigned seen = __ballot_sync(0xffffffffu, valid);
-        const int g0 = seen ? (__ffs(seen) - 1) >> 2 : 8, g1 = seen ? (31 - __clz(seen)) >> 2 : -1;
+        const bool whole = seen == 0xffffffffu;
+        const int first = seen ? __ffs(seen) - 1 : 32, last = seen ? 31 - __clz(seen) : -1;
         // scores: a group of four keys a pass, eight lanes a key
         float s = 0.f;
-#pragma unroll 2
-        for (int pass = g0; pass <= g1; ++pass) {
+        auto score = [&](int pass) {
             const int key = pass * 4 + (lane >> 3);
             const float4* k4 = reinterpret_cast<const float4*>(__shfl_sync(0xffffffffu, k_at, key));
             const int ksw = __shfl_sync(0xffffffffu, sw, key);
@@ -219,6 +225,13 @@ __global__ void __launch_bounds__(PF_WARPS * 32) attention_f32_kernel(AttentionA
             d += __shfl_xor_sync(0xffffffffu, d, 4);
             const float mine = __shfl_sync(0xffffffffu, d, (lane & 3) * 8);      // key pass * 4 + (lane & 3)
             if ((lane >> 2) == pass) s = mine;
+        };
+        if (whole) {
+#pragma unroll 2
+            for (int pass = 0; pass < 8; ++pass) score(pass);
+        } else {
+#pragma unroll 2
+            for (int pass = first >> 2; pass <= last >> 2; ++pass) score(pass);
         }
         s *= a.score_scale;
         if (a.softcap > 0.f) s = a.softcap * tanhf(s / a.softcap);
@@ -235,25 +248,54 @@ __global__ void __launch_bounds__(PF_WARPS * 32) attention_f32_kernel(AttentionA
 #pragma unroll
             for (int c = 0; c < VC; ++c) { acc[c].x *= corr; acc[c].y *= corr; acc[c].z *= corr; acc[c].w *= corr; }
         }
-#pragma unroll 2
-        for (int pass = g0; pass <= g1; ++pass) {
+        // values: the visible places in turn, whole warps
+        auto add = [](float4& sum, float w, const float4& v) {
+            sum.x = fmaf(w, v.x, sum.x);
+            sum.y = fmaf(w, v.y, sum.y);
+            sum.z = fmaf(w, v.z, sum.z);
+            sum.w = fmaf(w, v.w, sum.w);
+        };
+        auto value = [&](int key) {
+            const float pw = __shfl_sync(0xffffffffu, pj, key);
+            const float4* v4 = reinterpret_cast<const float4*>(__shfl_sync(0xffffffffu, v_at, key));
+            const int vsw = __shfl_sync(0xffffffffu, sw, key);
 #pragma unroll
-            for (int i4 = 0; i4 < 4; ++i4) {
-                const int key = pass * 4 + i4;
-                const float pw = __shfl_sync(0xffffffffu, pj, key);
-                const float4* v4 = reinterpret_cast<const float4*>(__shfl_sync(0xffffffffu, v_at, key));
-                const int vsw = __shfl_sync(0xffffffffu, sw, key);
-                if (!v4) continue;                          // uniform over the warp: a position that is not seen
-#pragma unroll
-                for (int c = 0; c < VC; ++c) {
-                    const int i = 32 * c + lane;
-                    const float4 v = i < chunks ? v4[vsw < 0 ? i : rdl_swizzled_chunk(vsw, i, chunks)] : zero4;
-                    acc[c].x = fmaf(pw, v.x, acc[c].x);
-                    acc[c].y = fmaf(pw, v.y, acc[c].y);
-                    acc[c].z = fmaf(pw, v.z, acc[c].z);
-                    acc[c].w = fmaf(pw, v.w, acc[c].w);
-                }
+            for (int c = 0; c < VC; ++c) {
+                const int i = 32 * c + lane;
+                const float4 v = i < chunks ? v4[vsw < 0 ? i : rdl_swizzled_chunk(vsw, i, chunks)] : zero4;
+                add(acc[c], pw, v);
             }
+        };
+        if (whole) {
+#pragma unroll 8
+            for (int key = 0; key < 32; ++key) value(key);
+        } else if constexpr (VC == 1) {
+            // eight loads at a time to the end: what is left over does not come one by one (places beyond the last add 0 * 0)
+#pragma unroll 1
+            for (int key0 = first; key0 <= last; key0 += 8) {
+                float4 v[8];
+                float pw[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const int key = key0 + u;
+                    const bool there = key <= last;
+                    const float w = __shfl_sync(0xffffffffu, pj, key);
+                    const float4* v4 = reinterpret_cast<const float4*>(__shfl_sync(0xffffffffu, v_at, key));
+                    const int vsw = __shfl_sync(0xffffffffu, sw, key);
+                    v[u] = there && lane < chunks ? v4[vsw < 0 ? lane : rdl_swizzled_chunk(vsw, lane, chunks)] : zero4;
+                    pw[u] = there ? w : 0.f;
+                }
+#pragma unroll
+                for (int u = 0; u < 8; ++u) add(acc[0], pw[u], v[u]);
+            }
+        } else {
+            int key = first;
+#pragma unroll 2
+            for (; key + 3 <= last; key += 4) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) value(key + u);
+            }
+            for (; key <= last; ++key) value(key);
         }
     }
 #pragma unroll

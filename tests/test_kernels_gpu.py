@@ -437,6 +437,23 @@ def test_float32_attention_of_short_and_ragged_contexts(window):
     assert_close(got, want, torch.float32, what="float32 attention", f32_tol=c.max_total * 2.0 ** -24)     # sums over the keys
 
 
+@pytest.mark.parametrize("window", [None, 7, 300])
+@pytest.mark.parametrize("head_dim", [24, 64, 100, 128, 200, 512])      # a value row of a lane's 16 bytes or several, whole and not
+def test_float32_attention_of_whole_and_partial_blocks(head_dim, window):
+    """A warp's 32 of 256 positions all visible, all but a few, a few and none; rows of the cache that no query sees hold NaN."""
+    past = [0, 1, 30, 33, 130, 222, 226, 229, 250, 255, 256, 257, 511, 700]
+    c = Case(dtype=torch.float32, seed=35, past=past, new=[270] + [1] * (len(past) - 2) + [3], n_heads=2, n_kv_heads=1, head_dim=head_dim, page_size=16, window=None)
+    c.window = window
+    b = c.batch("past")
+    want = ref.attention_vectorised(c.qkv, b, c.pages, new_kv=c.new_kv(), **c.kw(softcap=5.0))
+    unseen = [(row[j // 16], j % 16) for p, row in zip(past, c.pages.tables.tolist()) for j in range(c.max_total) if j >= p or (window and j <= p - window)]
+    pages, rows = (torch.tensor(i, device=DEV) for i in zip(*unseen))
+    for cache in (c.k, c.v):
+        cache[pages, :, rows] = math.nan
+    got = ops.attention(c.qkv, b, c.pages, new_kv=c.new_kv(), kind="plain", **c.kw(softcap=5.0))
+    assert_close(got, want, torch.float32, what="float32 attention", f32_tol=c.max_total * 2.0 ** -24)     # sums over the keys
+
+
 @pytest.mark.parametrize("head_dim,n_heads,n_kv_heads,page_size,window,chunk", [
     (256, 8, 4, 64, None, None), (256, 6, 3, 64, 300, None), (80, 8, 2, 48, None, None), (128, 8, 8, 128, None, 150), (64, 8, 1, 64, None, None),
     (32, 8, 4, 16, 200, None), (16, 8, 4, 64, None, None)])
