@@ -332,7 +332,6 @@ cudaError_t dc_launch_scan(const RecurrenceArgs* a, const float* records, cudaSt
 template <typename T, int RPS>
 int dc_launch(const RecurrenceArgs* a, float* records, int max_groups, cudaStream_t st) {
     RDL_CHECK_EX(rdl_launch(dc_record_kernel<T, RPS>, dim3(max_groups, a->n_heads), dim3(128), 0, st, *a, records), "delta_rule_chunked (records)");
-    const char* ev = getenv("RDL_X_CPL");
     // Two columns a lane halve the reads of a group's vectors from shared memory, which bound the walk where blocks share a
     // multiprocessor; with one block each the walk is bound by its own chain, which two columns lengthen.  Two blocks of one
     // column fit a multiprocessor.  Both launches, 16 heads of 128 x 128, one column against two: 1 x 1,500 tokens 506 / 610 us, 2 x 700

@@ -1,6 +1,8 @@
 """The engine's host logic (packing, paging, rings, slots, schedules) on a machine without a GPU:
 the CUDA entry points are replaced by the plain functions of tests/kernel_refs.py, everything
 above them is the product's code.  Logits are compared with the plain implementation."""
+import os
+
 import numpy as np
 import pytest
 import torch
@@ -10,6 +12,7 @@ import plain_gemma2 as plain
 import tiny_configs
 from rust_deeplearning_b200.config.base import architecture_for
 from rust_deeplearning_b200.engine.step import Engine
+from rust_deeplearning_b200.kernels import library
 from rust_deeplearning_b200.parts.model import Model
 from rust_deeplearning_b200.weights.loader import load_weights
 from rust_deeplearning_b200.weights.random_init import write_random_model
@@ -238,6 +241,15 @@ def test_prompt_attention_blocks_follow_the_keys_and_the_room():
     assert [blocks(p, 256, 700, 1) for p in (16, 17, 32, 33, 74, 75)] == [8, 4, 4, 2, 2, 1]        # its memory leaves room for one
     assert [blocks(p, 64, 700) for p in (32, 64, 65, 148)] == [8, 4, 1, 1]
     assert [blocks(p, 16, 45) for p in (64, 65)] == [4, 1]
+
+
+def test_no_launch_reads_the_environment():
+    """A launcher runs on every step: what the environment may set is read once, into a static."""
+    folder = os.path.dirname(os.path.abspath(library.__file__)) + "/../csrc/"
+    for f in sorted(os.listdir(folder)):
+        with open(folder + f, encoding="utf-8") as fh:
+            for line in fh:
+                assert "getenv" not in line or line.strip().startswith("static const"), (f, line)
 
 
 def test_what_a_device_needs_raised_is_raised_on_every_device(tmp_path):
