@@ -11,7 +11,7 @@ extern "C" {
 #define RDL_ACT_SILU 1
 #define RDL_ACT_SWISH_LIMIT 2   // min(g, L) sigmoid(1.702 min(g, L)) (clamp(u, -L, L) + 1), L a parameter
 
-#define RDL_ABI_VERSION 23
+#define RDL_ABI_VERSION 24
 
 const char* rdl_last_error(void);
 int rdl_abi_version(void);
@@ -321,7 +321,9 @@ int rdl_state_space_chunked(const RecurrenceArgs* a, void* work, long long work_
 long long rdl_state_space_chunked_work_bytes(int n_tokens, int n_seqs, int n_heads, int dim, int vdim);
 // The delta rule eight tokens at a time, in float (csrc/delta_rule_chunked.cu): heads of up to 128 key channels; two launches;
 // work: float scratch of rdl_delta_rule_chunked_work_bytes bytes, 16-byte aligned.
-int rdl_delta_rule_chunked(const RecurrenceArgs* a, void* work, long long work_bytes, void* stream);
+// longest: the most tokens a sequence of the step brings (0: not known); speed hangs on it, the result does not.
+int rdl_delta_rule_chunked(const RecurrenceArgs* a, int longest, void* work, long long work_bytes, void* stream);
+int rdl_delta_rule_columns(int n_tokens, int n_seqs, int longest, int n_heads, int vdim, int sms);
 long long rdl_delta_rule_chunked_work_bytes(int n_tokens, int n_seqs, int n_heads, int dim, int vdim);
 typedef struct {
     int dtype, bias_dtype;

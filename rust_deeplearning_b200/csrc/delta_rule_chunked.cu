@@ -330,13 +330,9 @@ cudaError_t dc_launch_scan(const RecurrenceArgs* a, const float* records, cudaSt
 }
 
 template <typename T, int RPS>
-int dc_launch(const RecurrenceArgs* a, float* records, int max_groups, cudaStream_t st) {
+int dc_launch(const RecurrenceArgs* a, int longest, float* records, int max_groups, cudaStream_t st) {
     RDL_CHECK_EX(rdl_launch(dc_record_kernel<T, RPS>, dim3(max_groups, a->n_heads), dim3(128), 0, st, *a, records), "delta_rule_chunked (records)");
-    // Two columns a lane halve the reads of a group's vectors from shared memory, which bound the walk where blocks share a
-    // multiprocessor; with one block each the walk is bound by its own chain, which two columns lengthen.  Two blocks of one
-    // column fit a multiprocessor.  Both launches, 16 heads of 128 x 128, one column against two: 1 x 1,500 tokens 506 / 610 us, 2 x 700
-    // (256 blocks) 262 / 305, 4 x 400 (512) 299 / 203, 16 x 100 303 / 211, 64 x 60 850 / 596, 200 + 633 + 1,066 + 1,500 810 / 634.
-    const bool two = (long long)a->n_seqs * a->n_heads * ((a->vdim + DC_COLS - 1) / DC_COLS) > 2 * rdl_sm_count();
+    const bool two = rdl_delta_rule_columns(a->n_tokens, a->n_seqs, longest, a->n_heads, a->vdim, rdl_sm_count()) == 2;
     RDL_CHECK_EX((two ? dc_launch_scan<RPS, 2>(a, records, st) : dc_launch_scan<RPS, 1>(a, records, st)), "delta_rule_chunked (scan)");
     return 0;
 }
@@ -349,7 +345,29 @@ extern "C" long long rdl_delta_rule_chunked_work_bytes(int n_tokens, int n_seqs,
     return (long long)dc_max_groups(n_tokens, n_seqs) * n_heads * rec * (long long)sizeof(float);
 }
 
-extern "C" int rdl_delta_rule_chunked(const RecurrenceArgs* a, void* work, long long work_bytes, void* stream) {
+// Columns of the state a lane of the second launch takes: 1 or 2.  longest: the most tokens a sequence of the step brings (0: not
+// known, all alike).
+//
+// Two columns halve the reads of a group's vectors from shared memory, which bound the walk where blocks wait for room (two of one
+// column find it on a multiprocessor: by shared memory with 65 to 128 key channels, by registers with fewer); a sequence that walks
+// alone they make slower.  So two where the blocks of one column do not all find room, and where what walks beside the longest
+// sequence (T / longest sequences like it) fills 0.85 of the room too; a sequence whose blocks take less than half of the
+// multiprocessors gains by two in any company.  Both launches, one column against two, microseconds (* what the rule takes):
+//   16 heads of 128 x 128    1 x 1,500 tokens 503* / 590    2 x 700 258* / 300    3 x 1,000 554 / 448*    4 x 400 294 / 196*    64 x 60 832 / 590*
+//       200 + 633 + 1,066 + 1,500 tokens 773 / 610*    1,500 + 1,000 + 500 666 / 629*    1,500 + 600 + 300 608* / 613    1,500 + 2 x 10 509* / 590
+//       1,500 + 7 x 10 531* / 601    2 x 1,500 + 2 x 100 617 / 635*    1,000 + 20 x 30 487* / 476    800 + 16 x 100 579 / 474*
+//   16 heads of 128 x 64     1 x 1,500 497* / 582    3 x 1,000 379* / 437    5 x 300 184 / 152*    1,500 + 7 x 10 507 / 353*    800 + 16 x 100 402 / 369*
+//   32 heads of 64 x 64      1 x 1,500 217* / 266    3 x 1,000 387 / 344*    20 x 100 271 / 212*    1,500 + 2 x 10 335* / 420    1,500 + 7 x 10 351* / 430
+// (These launches' blocks share multiprocessors, two each, while others stay idle: they start while the first launch's last blocks
+// hold room.  With room for one block only, 1 x 1,500 tokens of 16 heads of 128 x 128 took 304 / 347 us, but 3 x 1,000 606 / 489.)
+extern "C" int rdl_delta_rule_columns(int n_tokens, int n_seqs, int longest, int n_heads, int vdim, int sms) {
+    const long long each = (long long)n_heads * ((vdim + DC_COLS - 1) / DC_COLS), room = 2LL * sms;       // a sequence's blocks of one column
+    if (n_seqs * each <= room) return 1;
+    if (longest <= 0 || 2 * each <= sms) return 2;
+    return (double)n_tokens * each > 0.85 * (double)room * longest ? 2 : 1;
+}
+
+extern "C" int rdl_delta_rule_chunked(const RecurrenceArgs* a, int longest, void* work, long long work_bytes, void* stream) {
     RDL_REQUIRE(rdl_valid_dtype(a->dtype) && a->mode == RDL_REC_DELTA, "delta_rule_chunked: the delta rule only");
     RDL_REQUIRE(a->n_tokens >= 0 && a->n_seqs >= 0 && a->n_heads > 0 && a->n_key_heads > 0 && a->n_heads % a->n_key_heads == 0 && a->vdim > 0,
                 "delta_rule_chunked: bad sizes");
@@ -363,6 +381,7 @@ extern "C" int rdl_delta_rule_chunked(const RecurrenceArgs* a, void* work, long 
     const int max_groups = dc_max_groups(a->n_tokens, a->n_seqs);
     cudaStream_t st = (cudaStream_t)stream;
     float* records = (float*)work;
-    if (a->dtype == RDL_BF16) return a->dim <= 64 ? dc_launch<__nv_bfloat16, 4>(a, records, max_groups, st) : dc_launch<__nv_bfloat16, 8>(a, records, max_groups, st);
-    return a->dim <= 64 ? dc_launch<float, 4>(a, records, max_groups, st) : dc_launch<float, 8>(a, records, max_groups, st);
+    if (a->dtype == RDL_BF16)
+        return a->dim <= 64 ? dc_launch<__nv_bfloat16, 4>(a, longest, records, max_groups, st) : dc_launch<__nv_bfloat16, 8>(a, longest, records, max_groups, st);
+    return a->dim <= 64 ? dc_launch<float, 4>(a, longest, records, max_groups, st) : dc_launch<float, 8>(a, longest, records, max_groups, st);
 }

@@ -89,6 +89,7 @@ class StepBatch:
     shared_runs: frozenset = frozenset()                             # runs whose keys and values a later run reads
     status: Optional[torch.Tensor] = None                            # int32 flag kernels set when they give up a wait
     has_past: bool = True                                            # some sequence of the step has earlier positions in the cache
+    longest_new: int = 0                                             # the most new tokens of a sequence (0: not known)
 
     def attention_batch(self, keys_in_cache: str, window: Optional[int] = None) -> AttentionBatch:
         """keys_in_cache: "past" - new keys are read from the step's packed rows;

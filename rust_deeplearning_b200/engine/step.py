@@ -162,6 +162,7 @@ class Engine:
                                       is_decode=is_decode, max_total_len=max(totals), scratch=self._scratch)
             batch.status = self.status
             batch.has_past = max(past) > 0
+            batch.longest_new = max(lens)
             logits = self._forward(batch)
             self.eager_steps += 1
         self.cache.advance(slots, lens)

@@ -23,7 +23,7 @@ from concurrent.futures import ThreadPoolExecutor
 _PKG = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(_PKG, "csrc")
 LIB_NAME = "librdl_b200_kernels.so"
-ABI_VERSION = 23
+ABI_VERSION = 24
 
 # fast math is never enabled: the 32-bit path relies on exact tanhf/expf/sqrtf and plain FMA
 NVCC_FLAGS = ["-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
@@ -418,7 +418,8 @@ _SIGNATURES = {
     "rdl_recurrence_scan": [ctypes.POINTER(RecurrenceArgs), _P],
     "rdl_delta_prepare": [ctypes.POINTER(DeltaPrepareArgs), _P],
     "rdl_state_space_chunked": [ctypes.POINTER(RecurrenceArgs), _P, _LL, _P],
-    "rdl_delta_rule_chunked": [ctypes.POINTER(RecurrenceArgs), _P, _LL, _P],
+    "rdl_delta_rule_chunked": [ctypes.POINTER(RecurrenceArgs), _I, _P, _LL, _P],
+    "rdl_delta_rule_columns": [_I, _I, _I, _I, _I, _I],
     "rdl_decay_attention_scan": [ctypes.POINTER(DecayAttentionArgs), _P],
     "rdl_decay_attention_chunked": [ctypes.POINTER(DecayAttentionArgs), _P, _LL, _P],
     "rdl_decay_attention_chunks": [_I, _I],

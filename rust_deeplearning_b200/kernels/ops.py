@@ -1742,14 +1742,15 @@ def delta_prepare(rows: torch.Tensor, *, q_col: int, k_col: int, n_heads: int, n
 
 
 def delta_rule_scan(rows: torch.Tensor, *, v_col: int, q_f, k_f, g_f, beta_f, n_heads: int, n_key_heads: int, dim: int, vdim: int,
-                    state: torch.Tensor, tok_pos, seq_start, slots, n_seqs: int, kind: str = "auto") -> torch.Tensor:
+                    state: torch.Tensor, tok_pos, seq_start, slots, n_seqs: int, longest: int = 0, kind: str = "auto") -> torch.Tensor:
     """The delta rule with a decay per key channel, in float: per head h with key head j(h),
     S <- g_t (.) S (row i times g_t[i]);  u = beta_t (v_t - S^T k_t);  S <- S + k_t u^T;  o_t = S^T q_t,
     v [vdim] of head h from column v_col of `rows`, the rest as `delta_prepare` made it; S float32 [slots, heads, dim, vdim]
     read from and left in `state`.  Returns float32 [tokens, heads * vdim].
     kind: "scan" (token by token), "chunked" (eight tokens at a time: what depends on no state is made for all groups at
     once, the state takes a group's writes in one pass; heads of up to 128 key channels), "auto" (groups where sequences
-    bring many bfloat16 tokens each)."""
+    bring many bfloat16 tokens each).  longest: the most tokens a sequence of the step brings, where the caller knows it (the
+    chunked kernels divide their work by it; the result does not hang on it)."""
     a = library.RecurrenceArgs()
     out = _recurrence_common(a, rows, state, n_heads, n_key_heads, dim, vdim, tok_pos, seq_start, slots, n_seqs)
     T = rows.shape[0]
@@ -1769,7 +1770,7 @@ def delta_rule_scan(rows: torch.Tensor, *, v_col: int, q_f, k_f, g_f, beta_f, n_
         _need(dim <= DELTA_CHUNKED_MAX_DIM, f"delta_rule_scan: the chunked kernels take heads of up to {DELTA_CHUNKED_MAX_DIM} key channels")
         nbytes = lib.rdl_delta_rule_chunked_work_bytes(T, n_seqs, n_heads, dim, vdim)
         work = torch.empty((nbytes // 4,), dtype=torch.float32, device=rows.device)
-        library.check(lib.rdl_delta_rule_chunked(ctypes.byref(a), _ptr(work), nbytes, _stream(rows)), 2)
+        library.check(lib.rdl_delta_rule_chunked(ctypes.byref(a), longest, _ptr(work), nbytes, _stream(rows)), 2)
     else:
         raise KernelError(f"delta_rule_scan: unknown kind '{kind}'")
     return out

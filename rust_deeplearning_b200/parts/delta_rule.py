@@ -69,7 +69,7 @@ class DeltaRule:
                                                   decay_rows=wide[:, :H * d], beta_rows=rows[:, self.b_col:self.b_col + H],
                                                   dt_bias=self.dt_bias, a_log=self.a_log, q_scale=self.q_scale, unit_eps=self.unit_eps)
         o = ops.delta_rule_scan(qkv, v_col=2 * J * d, q_f=q_f, k_f=k_f, g_f=g_f, beta_f=beta_f, n_heads=H, n_key_heads=J, dim=d,
-                                vdim=e, state=cache.state[0], n_seqs=batch.n_seqs, **where)
+                                vdim=e, state=cache.state[0], n_seqs=batch.n_seqs, longest=batch.longest_new, **where)
         y = ops.group_norm_gate(o, H, eps=self.eps, weight=self.norm_weight, gate=wide[:, H * d:], gate_kind="sigmoid", out_dtype=x.dtype)
         return ops.linear(y, self.w_o)
 

@@ -243,6 +243,22 @@ def test_prompt_attention_blocks_follow_the_keys_and_the_room():
     assert [blocks(p, 16, 45) for p in (64, 65)] == [4, 1]
 
 
+def test_delta_rule_columns_follow_the_walk(tmp_path, monkeypatch):
+    """Two columns a lane where the tokens fill the chip beside the longest sequence, not where sequences of a few tokens stand beside it;
+    the engine says how long the longest is."""
+    columns = lambda lens, heads=16, vdim=128: library.load().rdl_delta_rule_columns(sum(lens), len(lens), max(lens), heads, vdim, 148)
+    assert [columns(x) for x in ([1500], [700] * 2, [1500, 10, 10], [1500] + [10] * 7, [10] * 7 + [1500], [1500, 600, 300])] == [1] * 6
+    assert [columns(x) for x in ([1000] * 3, [400] * 4, [60] * 64, [200, 633, 1066, 1500], [1500, 1000, 500], [800] + [100] * 16)] == [2] * 6
+    assert [columns([n] * 9, 2, 256) for n in (1, 10 ** 6)] == [1, 1] and [columns([n] * 10, 2, 256) for n in (1, 10 ** 6)] == [2, 2]
+    assert [columns([1500] + [10] * n, vdim=64) for n in (3, 4)] == [1, 2]          # its own blocks take less than half of the chip
+    assert library.load().rdl_delta_rule_columns(1570, 8, 0, 16, 128, 148) == 2     # not known
+    engine, _, _ = build(tmp_path, "A", monkeypatch)
+    seen, forward = [], engine._forward
+    monkeypatch.setattr(engine, "_forward", lambda batch: seen.append(batch.longest_new) or forward(batch))
+    engine.step([engine.new_sequence() for _ in range(3)], [[1, 2], [3] * 9, [4]])
+    assert seen == [9]
+
+
 def test_no_launch_reads_the_environment():
     """A launcher runs on every step: what the environment may set is read once, into a static."""
     folder = os.path.dirname(os.path.abspath(library.__file__)) + "/../csrc/"
