@@ -191,8 +191,10 @@ cudaError_t launch_few_rows(float* out, const float* x, const float* w, int M, i
 // ---- many rows ----
 
 constexpr int TN = 8, BN = 16 * TN;
-// Blocks a multiprocessor: what the registers of 16 TY threads with 8 TM sums each allow.
-__host__ __device__ constexpr int tile_blocks(int tm, int ty) { return ty == 8 ? (tm <= 6 ? 3 : 2) : (tm <= 4 ? 2 : 1); }
+// Blocks a multiprocessor: what the registers of 16 TY threads with 8 TM sums each and a ring of so many chunks leave room for.  (Forms
+// of three chunks held to the 168 registers of three blocks spilled 12 to 40 bytes for it: 32 rows 16.9 us against 15.5 for up to
+// 15 tiles of 2,304 terms, 25.2 against 24.5 for 32 tiles.)
+__host__ __device__ constexpr int tile_blocks(int tm, int ty, int chunks) { return ty == 16 || chunks == 5 ? 1 : tm <= 6 && chunks == 2 ? 3 : 2; }
 
 __device__ __forceinline__ uint32_t f32_cluster_rank() {
     uint32_t r;
@@ -213,7 +215,7 @@ __device__ __forceinline__ float f32_ld_remote(uint32_t addr, uint32_t rank) {
 // A tile of TY TM rows by 128 columns; thread (ty, tx) has rows ty + TY i and columns tx + 16 j.  SHARED: the block is one of a
 // cluster of eight along z, each with a run of k.
 template <int TM, int TY, int TILE_STAGES, bool SHARED, bool ALIGNED>
-__global__ void __launch_bounds__(16 * TY, tile_blocks(TM, TY)) gemm_f32_tile_kernel(float* __restrict__ out, const float* __restrict__ x,
+__global__ void __launch_bounds__(16 * TY, tile_blocks(TM, TY, TILE_STAGES)) gemm_f32_tile_kernel(float* __restrict__ out, const float* __restrict__ x,
                                                                             const float* __restrict__ w, int M, int N, int K) {
     constexpr int BM = TY * TM, STAGE = (BM + BN) * PITCH, RP = 2 * TY;      // RP: rows a pass of copies takes
            // STAGE: floats
@@ -356,7 +358,7 @@ cudaError_t launch_tile_rows(float* out, const float* x, const float* w, int M, 
     // of eight reach about seven eighths of the multiprocessors, and their meeting costs about as much again).
     constexpr int WHOLE = TY == 16 ? 3 : 2;                       // chunks of the ring with as many blocks as a multiprocessor takes
     const long long tiles = (long long)((N + BN - 1) / BN) * ((M + TY * TM - 1) / (TY * TM)), blocks8 = tiles * RUNS;
-    const long long sms8 = rdl_sm_count() * 7LL / 8, slots = (long long)rdl_sm_count() * tile_blocks(TM, TY), slots8 = sms8 * tile_blocks(TM, TY);
+    const long long sms8 = rdl_sm_count() * 7LL / 8, slots = (long long)rdl_sm_count() * tile_blocks(TM, TY, WHOLE), slots8 = sms8 * tile_blocks(TM, TY, WHOLE);
     const double whole = (double)((tiles + slots - 1) / slots), eighths = (double)((blocks8 + slots8 - 1) / slots8) / RUNS * 1.15;
     if (whole <= eighths) return launch_tile<TM, TY, WHOLE, false, ALIGNED>(out, x, w, M, N, K, st);
     // A shared tile's run of k is a few chunks long, and fewer blocks on a multiprocessor hide less of the wait for them: a deeper
