@@ -194,7 +194,10 @@ constexpr int TN = 8, BN = 16 * TN;
 // Blocks a multiprocessor: what the registers of 16 TY threads with 8 TM sums each and a ring of so many chunks leave room for.  (Forms
 // of three chunks held to the 168 registers of three blocks spilled 12 to 40 bytes for it: 32 rows 16.9 us against 15.5 for up to
 // 15 tiles of 2,304 terms, 25.2 against 24.5 for 32 tiles.)
-__host__ __device__ constexpr int tile_blocks(int tm, int ty, int chunks) { return ty == 16 || chunks == 5 ? 1 : tm <= 6 && chunks == 2 ? 3 : 2; }
+__host__ __device__ constexpr int tile_blocks(int tm, int ty, int chunks) { return ty == 16 ? 1 : tm <= 6 && chunks == 2 ? 3 : 2; }
+// Clusters of eight blocks that find room at once with 1, 2 or 3 blocks a multiprocessor: 15, 33 and 48 of 148 multiprocessors (the
+// runtime's occupancy query; a cluster lies inside one group of multiprocessors, and not every group's number is a multiple of eight).
+constexpr long long clusters_at(int blocks, int sms) { return (blocks == 1 ? 15LL : blocks == 2 ? 33LL : 48LL) * sms / 148; }
 
 __device__ __forceinline__ uint32_t f32_cluster_rank() {
     uint32_t r;
@@ -217,8 +220,8 @@ __device__ __forceinline__ float f32_ld_remote(uint32_t addr, uint32_t rank) {
 template <int TM, int TY, int TILE_STAGES, bool SHARED, bool ALIGNED>
 __global__ void __launch_bounds__(16 * TY, tile_blocks(TM, TY, TILE_STAGES)) gemm_f32_tile_kernel(float* __restrict__ out, const float* __restrict__ x,
                                                                             const float* __restrict__ w, int M, int N, int K) {
-    constexpr int BM = TY * TM, STAGE = (BM + BN) * PITCH, RP = 2 * TY;      // RP: rows a pass of copies takes
-           // STAGE: floats
+    constexpr int BM = TY * TM, STAGE = (BM + BN) * PITCH, RP = 2 * TY;      // STAGE: floats of a chunk; RP: rows a pass of copies takes
+    static_assert(BM % RP == 0 && BN % RP == 0, "whole passes of copies");
     extern __shared__ __align__(16) float sm[];
     float* sums = sm + TILE_STAGES * STAGE;                       // [BM][BN]: the runs' sums so far (SHARED: this block's run)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -238,9 +241,8 @@ __global__ void __launch_bounds__(16 * TY, tile_blocks(TM, TY, TILE_STAGES)) gem
             }
         } else {
 #pragma unroll
-            for (int i = 0; i < (BM + RP - 1) / RP; ++i) {
+            for (int i = 0; i < BM / RP; ++i) {
                 const int r = i * RP + (tid >> 3), kk = k + (tid & 7) * 4, m = m0 + r;
-                if (BM % RP && r >= BM) continue;
                 const bool ok = m < M && kk < k_hi;
                 copy4<ALIGNED>(base + (uint32_t)((s * STAGE + r * PITCH + (tid & 7) * 4) * 4), ok ? x + (long long)m * K + kk : x, ok ? k_hi - kk : 0);
             }
@@ -351,49 +353,81 @@ cudaError_t launch_tile(float* out, const float* x, const float* w, int M, int N
     return cudaLaunchKernelEx(&cfg, gemm_f32_tile_kernel<TM, TY, STAGES, SHARED, ALIGNED>, out, x, w, M, N, K);
 }
 
-template <int TM, int TY, bool ALIGNED>
-cudaError_t launch_tile_rows(float* out, const float* x, const float* w, int M, int N, int K, cudaStream_t st) {
-    // (the rule's other sides are measured beside launch_rows)
-    // Eight blocks a tile where the waves of whole tiles would leave more of the chip idle than the eighths' waves do (clusters
-    // of eight reach about seven eighths of the multiprocessors, and their meeting costs about as much again).
-    constexpr int WHOLE = TY == 16 ? 3 : 2;                       // chunks of the ring with as many blocks as a multiprocessor takes
-    const long long tiles = (long long)((N + BN - 1) / BN) * ((M + TY * TM - 1) / (TY * TM)), blocks8 = tiles * RUNS;
-    const long long sms8 = rdl_sm_count() * 7LL / 8, slots = (long long)rdl_sm_count() * tile_blocks(TM, TY, WHOLE), slots8 = sms8 * tile_blocks(TM, TY, WHOLE);
-    const double whole = (double)((tiles + slots - 1) / slots), eighths = (double)((blocks8 + slots8 - 1) / slots8) / RUNS * 1.15;
-    if (whole <= eighths) return launch_tile<TM, TY, WHOLE, false, ALIGNED>(out, x, w, M, N, K, st);
-    // A shared tile's run of k is a few chunks long, and fewer blocks on a multiprocessor hide less of the wait for them: a deeper
-    // ring where the clusters leave room for it (4,096 outputs of 2,304, 48 rows, 256 blocks: 42 us with two chunks, 33 with three.
-    // Where it takes a multiprocessor from a cluster it costs a second wave: 2,304 of 9,216, 144 blocks, 110 and, five chunks, 142).
-    if constexpr (TY == 8) {
-        if (blocks8 <= sms8) return launch_tile<TM, TY, 5, true, ALIGNED>(out, x, w, M, N, K, st);
-        if constexpr (TM <= 6) {
-            if (4 * blocks8 > 5 * sms8 && blocks8 <= 2 * sms8) return launch_tile<TM, TY, 3, true, ALIGNED>(out, x, w, M, N, K, st);
+// The form of a product of more than FEW_MAX rows: rows of a tile, chunks of the ring, and whether eight blocks share a tile.
+struct TileForm { int rows, chunks; bool shared; };
+
+// What a wave of tiles costs by the blocks a multiprocessor holds of it (1, 2, 3), and a further wave behind full ones, in
+// microseconds for eighths of 9,216 terms; a wave of whole tiles costs eight times its entry.  Measured with 2,304 to 28,672 outputs of
+// 2,048 to 14,336 terms and 32 to 2,048 rows.  (Whole tiles of 48 rows fill multiprocessors with three while others hold one.)
+struct TileCost { int rows, levels, shared[3], shared_on, whole[3], whole_on; };
+constexpr TileCost TILE_COSTS[] = {{32, 3, {51, 82, 113}, 105, {51, 83, 115}, 110},
+                                   {48, 3, {68, 110, 149}, 138, {69, 155, 165}, 153},
+                                   {64, 2, {81, 140, 0}, 134, {82, 141, 0}, 134},
+                                   {128, 1, {130, 0, 0}, 139, {132, 0, 0}, 138}};
+
+inline long long tile_cost(const TileCost& c, bool shared, long long tiles, int sms) {
+    auto room = [&](int blocks) { return shared ? clusters_at(blocks, sms) : (long long)blocks * sms; };
+    const long long full = room(c.levels) > 0 ? room(c.levels) : 1, before = (tiles - 1) / full, last = tiles - before * full;
+    int level = 1;
+    while (level < c.levels && last > room(level)) ++level;
+    return shared ? before * c.shared_on + c.shared[level - 1] : 8 * (before * c.whole_on + c.whole[level - 1]);
+}
+
+// The form whose waves cost least.  Of 244 products of 2,304 to 256,000 outputs and 20 to 2,048 rows it takes one within 5 % of the best
+// form in 238.  Microseconds by form, s: shared by eight blocks, * what is taken; in brackets what a rule on the rows alone took
+// (tiles of 32, 48 or 64 rows up to 96, then 64 or 128 by the multiprocessors that tiles of 128 give one):
+//   2,304 outputs of 9,216    32 rows  32s 83*   48 rows  32s 114  48s 109*   64 rows  32s 114* (138)  48s 155  64s 138    90 rows  32s 152  48s 155*  64s 205
+//                            120 rows  32s 194* (208)  48s 203  64s 207  128s 258     200 rows  32s 301  48s 306*  64s 334 (334)  128s 386
+//                            700 rows  48s 798* (1,129)  64s 814  64 1,131  128 1,053  128s 1,037
+//   18,432 outputs of 2,304   48 rows  32s 171  48s 121*  64s 164   64 rows  32s 171  64s 165*  64 173   120 rows  32 317  64 294  128 277*    900 rows  48 1,984* (2,199)
+//   3,584 outputs of 14,336   64 rows  32s 235  64s 212*   128 rows  32s 415  64s 429 (429)  128s 396*   160 rows  32s 509* (603)  64s 604   512 rows  48s 1,385* (1,753)  128 1,627
+//   8,192 outputs of 3,584    96 rows  48s 165*   256 rows  32s 441  64s 419  128 421* (449)   384 rows  48s 588* (697)  64s 622  128 838
+//   256 outputs of 96         64 rows  32s 4.1* (5.9)  64s 5.9
+// Where it errs the sums are short, so that the meeting of a shared tile weighs more: 5,000 outputs of 300, 400 rows 80 us against 73.
+inline TileForm tile_form(int M, int N, int sms) {
+    TileForm best = {0, 0, false};
+    long long least = 0;
+    for (const TileCost& c : TILE_COSTS) {
+        const long long down = ((long long)M + c.rows - 1) / c.rows, tiles = (N + (long long)BN - 1) / BN * down;
+        if (down > 65535 && c.rows < 64) continue;               // the grid's height
+        for (const bool shared : {true, false}) {
+            const long long cost = tile_cost(c, shared, tiles, sms);
+            if (best.rows && cost >= least) continue;
+            least = cost;
+            // Three chunks, which leave room for two blocks a multiprocessor, where all tiles find room in that way and with two chunks
+            // some multiprocessors would hold three blocks, others one (48 rows of 2,304 terms: 24 tiles 31.2 us with two chunks, 32.1
+            // with three; 25 tiles 41.2 and 32.1, 32 tiles 41.4 and 32.7; fewer tiles take 20 either way).  Five chunks and one block
+            // never won: up to 15 tiles 20 us, from 16 on, which are two waves, 38.
+            const bool three = c.rows == 128 || (c.rows < 64 && shared && 2 * tiles > clusters_at(3, sms) && tiles <= clusters_at(2, sms));
+            best = {c.rows, three ? 3 : 2, shared};
         }
     }
-    return launch_tile<TM, TY, WHOLE, true, ALIGNED>(out, x, w, M, N, K, st);
+    return best;
 }
 
 template <bool ALIGNED>
 cudaError_t launch_rows(float* out, const float* x, const float* w, int M, int N, int K, cudaStream_t st) {
     if (M <= FEW_MAX) return launch_few_rows<ALIGNED>(out, x, w, M, N, K, st);
-    // The tile height that pads least; from 97 rows on 128 where such tiles give nine tenths of the multiprocessors one and 128 pads by
-    // at most a tenth more than 64, else 64.  Microseconds by height, s: shared by eight blocks, * what the rules take; in brackets what
-    // tiles of half as many sums a thread (16 threads along the rows) took:
-    //   2,304 outputs of 9,216    32 rows  32s 84* (106)   48 rows  32s 115  48s 110* (125)  64s 140     64 rows  32s 115  48s 156  64s 140* (149)
-    //                             90 rows  32s 155  48s 156* (188)  64s 205    120 rows  32s 198  48s 204  64s 208* (258)  128s 258
-    //                            200 rows  32s 301  48s 308  64s 331* (387)  128s 387   256 rows  48s 348  64s 330* (388)  128s 388
-    //   18,432 outputs of 2,304   32 rows  32 109  32s 93* (125)   48 rows  32s 172  48 143  48s 122* (146)  64s 165     64 rows  64 173  64s 165* (172)
-    //                             90 rows  48s 227* (238)  64 294  128 275     120 rows  64 295  64s 314  128 278* (278)    200 rows  48s 539  128 550* (550)
-    //   4,096 outputs of 2,304    32 rows  32s 25* (31)   48 rows  48s 33* (35)   64 rows  32s 52  64s 40* (41)   90 rows  48s 67* (70)  120 rows  64s 78* (109)
-    //   256,000 outputs of 2,304  45 rows  48 1484* (1605)
-    if (M <= 32) return launch_tile_rows<4, 8, ALIGNED>(out, x, w, M, N, K, st);
-    if (M <= 48 || (M > 64 && M <= 96)) return launch_tile_rows<6, 8, ALIGNED>(out, x, w, M, N, K, st);
-    const long long p128 = (M + 127) / 128 * 128LL, p64 = (M + 63) / 64 * 64LL, tiles128 = (N + BN - 1) / BN * (p128 / 128);
-    return 10 * tiles128 < 9LL * rdl_sm_count() || 10 * p128 > 11 * p64 ? launch_tile_rows<8, 8, ALIGNED>(out, x, w, M, N, K, st)
-                                                                        : launch_tile_rows<8, 16, ALIGNED>(out, x, w, M, N, K, st);
+    const TileForm f = tile_form(M, N, rdl_sm_count());
+    if (f.rows == 32) return !f.shared ? launch_tile<4, 8, 2, false, ALIGNED>(out, x, w, M, N, K, st)
+                             : f.chunks == 2 ? launch_tile<4, 8, 2, true, ALIGNED>(out, x, w, M, N, K, st)
+                                             : launch_tile<4, 8, 3, true, ALIGNED>(out, x, w, M, N, K, st);
+    if (f.rows == 48) return !f.shared ? launch_tile<6, 8, 2, false, ALIGNED>(out, x, w, M, N, K, st)
+                             : f.chunks == 2 ? launch_tile<6, 8, 2, true, ALIGNED>(out, x, w, M, N, K, st)
+                                             : launch_tile<6, 8, 3, true, ALIGNED>(out, x, w, M, N, K, st);
+    if (f.rows == 64) return f.shared ? launch_tile<8, 8, 2, true, ALIGNED>(out, x, w, M, N, K, st) : launch_tile<8, 8, 2, false, ALIGNED>(out, x, w, M, N, K, st);
+    return f.shared ? launch_tile<8, 16, 3, true, ALIGNED>(out, x, w, M, N, K, st) : launch_tile<8, 16, 3, false, ALIGNED>(out, x, w, M, N, K, st);
 }
 
 }  // namespace
+
+// The form a product takes on so many multiprocessors: 100 x rows of a tile + 10 x chunks of the ring + 1 where eight blocks share a tile;
+// 0: the few-row kernel.
+extern "C" int rdl_gemm_f32_form(int m, int n, int sms) {
+    if (m <= FEW_MAX) return 0;
+    const TileForm f = tile_form(m, n, sms);
+    return 100 * f.rows + 10 * f.chunks + (f.shared ? 1 : 0);
+}
 
 extern "C" int rdl_gemm_f32(void* out, const void* x, const void* w, int m, int n, int k, void* stream) {
     RDL_REQUIRE(m >= 0 && n > 0 && k > 0, "gemm_f32: bad sizes m=%d n=%d k=%d", m, n, k);

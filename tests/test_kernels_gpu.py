@@ -9,7 +9,7 @@ import pytest
 import torch
 
 import kernel_refs as ref
-from rust_deeplearning_b200.kernels import ops
+from rust_deeplearning_b200.kernels import library, ops
 from rust_deeplearning_b200.sampling.sampler import uniform_for
 
 pytestmark = pytest.mark.gpu
@@ -115,8 +115,8 @@ def test_gemm_f32_sums_in_one_order_whatever_the_kernel(k):
 
 @pytest.mark.parametrize("k", [97, 100])
 def test_gemm_f32_sums_in_one_order_with_many_outputs(k):
-    """So many outputs that the tiles are not shared (at every height) and that few rows take tiles of 32 weight rows, the last ones
-    partial; on and off 16-byte boundaries.  The rows of 300, whose tiles are shared for the last columns alone, give the bits."""
+    """So many outputs that few rows take tiles of 32 weight rows, the last ones partial, and several waves of tiles of every height
+    above; on and off 16-byte boundaries.  The last columns alone, in tiles of another form, give the bits."""
     n, tail = 25001, 700
     x, w = rnd((300, k), torch.float32, k), rnd((n, k), torch.float32, 5)
     off = torch.empty(n * k + 1, dtype=torch.float32, device=w.device)[1:].view(n, k).copy_(w)
@@ -128,7 +128,7 @@ def test_gemm_f32_sums_in_one_order_with_many_outputs(k):
             assert torch.equal(ops.linear(x[:m].contiguous(), weight), full[:m]), (m, weight is off)
 
 
-@pytest.mark.parametrize("n", [1000, 4000, 5000, 60001])      # shared tiles with rings of five, three and two chunks; whole tiles
+@pytest.mark.parametrize("n", [1000, 4000, 5000, 60001])      # shared tiles with rings of two and of three chunks, in one wave and in several
 def test_gemm_f32_sums_in_one_order_at_every_ring_depth(n):
     """k of 300: runs of 40, the last one shorter, chunks that end early; rows on both sides of every tile height."""
     k, tail = 300, 130
@@ -139,6 +139,24 @@ def test_gemm_f32_sums_in_one_order_at_every_ring_depth(n):
     for m in (17, 32, 33, 48, 49, 64, 65, 96, 97, 128):
         for weight in (w, off):
             assert torch.equal(ops.linear(x[:m].contiguous(), weight), rows[:m]), (m, weight is off)
+
+
+@pytest.mark.parametrize("form", [3220, 3221, 3231, 4820, 4821, 4831, 6420, 6421, 12830, 12831])
+def test_gemm_f32_sums_in_one_order_in_every_form(form):
+    """Each form a product of more than 16 rows may take (rows of a tile, chunks, shared or whole), at the smallest of some sizes that takes it
+    on this device, gives the few-row kernel's bits in its first and last columns; weights on and off 16-byte boundaries."""
+    takes = library.load().rdl_gemm_f32_form
+    sizes = [(m, n) for m in (17, 31, 33, 47, 50, 64, 97, 127, 160, 200, 299) for n in (1000, 3500, 6000, 12001, 16001, 18000, 25001, 36001, 50001, 75001)
+             if takes(m, n, ops.sm_count(0)) == form]
+    assert sizes, form
+    (m, n), k = min(sizes, key=lambda s: s[0] * s[1]), 300
+    x, w = rnd((m, k), torch.float32, 3), rnd((n, k), torch.float32, n)
+    off = torch.empty(n * k + 1, dtype=torch.float32, device=w.device)[1:].view(n, k).copy_(w)
+    edges = torch.cat([w[:130], w[-130:]])
+    want = torch.cat([ops.linear(x[i:i + 10].contiguous(), edges) for i in range(0, m, 10)])
+    for weight in (w, off):
+        got = ops.linear(x, weight)
+        assert torch.equal(torch.cat([got[:, :130], got[:, -130:]], 1), want), (m, n, weight is off)
 
 
 def test_linear_bf16_float32_output():
