@@ -203,7 +203,9 @@ __device__ __forceinline__ float dc_sum16(const float (&x)[16], int r) {
     return mine + __shfl_xor_sync(full, send, 1);
 }
 
-// CPL: columns of a lane.
+// CPL: columns of a lane.  Two blocks a multiprocessor: with 65 to 128 key channels shared memory leaves room for no more; with fewer it
+// would for four, but the 64 registers these leave a thread cost more than the blocks bring (16 heads of 64 x 64, four blocks and
+// two: 1,500 tokens 579 / 192 us, 64 x 60 309 / 329 and with two columns 251 / 261).
 template <int RPS, int CPL>
 __global__ void __launch_bounds__(DC_THREADS, 2) dc_scan_kernel(RecurrenceArgs a, const float* __restrict__ records) {
     using R = DcRecord<RPS>;
