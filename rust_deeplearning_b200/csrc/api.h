@@ -11,7 +11,7 @@ extern "C" {
 #define RDL_ACT_SILU 1
 #define RDL_ACT_SWISH_LIMIT 2   // min(g, L) sigmoid(1.702 min(g, L)) (clamp(u, -L, L) + 1), L a parameter
 
-#define RDL_ABI_VERSION 24
+#define RDL_ABI_VERSION 25
 
 const char* rdl_last_error(void);
 int rdl_abi_version(void);
@@ -366,7 +366,7 @@ int rdl_decay_attention_chunked(const DecayAttentionArgs* a, void* work, long lo
 
 // out[m, n] = sum_k x[m, k] * w[n, k], all float, plain FMA in a fixed order of k
 int rdl_gemm_f32(void* out, const void* x, const void* w, int m, int n, int k, void* stream);
-int rdl_gemm_f32_form(int m, int n, int sms);      // 100 x rows of a tile + 10 x chunks + 1 where eight blocks share a tile; 0: few rows
+int rdl_gemm_f32_form(int m, int n, int k, int sms);      // 100 x rows of a tile + 10 x chunks + 1 where eight blocks share a tile; 0: few rows
 
 // out[m, n] = epilogue(sum_k x[m, k] * w[n, k]) for m <= 16, bfloat16 operands, float accumulation.
 // gated: w is [2 n, k] (gate rows, then up rows) and the result is act(gate) * up (or a gated form with a parameter,

@@ -365,33 +365,37 @@ constexpr TileCost TILE_COSTS[] = {{32, 3, {51, 82, 113}, 105, {51, 83, 115}, 11
                                    {64, 2, {81, 140, 0}, 134, {82, 141, 0}, 134},
                                    {128, 1, {130, 0, 0}, 139, {132, 0, 0}, 138}};
 
-inline long long tile_cost(const TileCost& c, bool shared, long long tiles, int sms) {
+// In microseconds: the waves, by the k their chunks hold, and for shared tiles what a wave's meeting costs beyond what long sums hide.
+inline double tile_cost(const TileCost& c, bool shared, long long tiles, int K, int sms) {
     auto room = [&](int blocks) { return shared ? clusters_at(blocks, sms) : (long long)blocks * sms; };
     const long long full = room(c.levels) > 0 ? room(c.levels) : 1, before = (tiles - 1) / full, last = tiles - before * full;
+    // (behind full waves the ring stays at two chunks: from half of a wave on some multiprocessors then hold three blocks)
+    auto fits = [&](int blocks) { return shared && before > 0 && blocks == 2 && c.levels == 3 ? room(3) / 2 : room(blocks); };
     int level = 1;
-    while (level < c.levels && last > room(level)) ++level;
-    return shared ? before * c.shared_on + c.shared[level - 1] : 8 * (before * c.whole_on + c.whole[level - 1]);
+    while (level < c.levels && last > fits(level)) ++level;
+    const double held = (double)RUNS * ((run_length(K) + KC - 1) / KC * KC) / 9216;
+    return shared ? held * (before * c.shared_on + c.shared[level - 1]) + 0.8 * (before + 1) : held * RUNS * (before * c.whole_on + c.whole[level - 1]);
 }
 
-// The form whose waves cost least.  Of 244 products of 2,304 to 256,000 outputs and 20 to 2,048 rows it takes one within 5 % of the best
-// form in 238.  Microseconds by form, s: shared by eight blocks, * what is taken; in brackets what a rule on the rows alone took
+// The form whose waves cost least.  Of 245 products of 96 to 28,672 outputs and 20 to 2,048 rows it takes one within 5 % of the best
+// form in 239.  Microseconds by form, s: shared by eight blocks, * what is taken; in brackets what a rule on the rows alone took
 // (tiles of 32, 48 or 64 rows up to 96, then 64 or 128 by the multiprocessors that tiles of 128 give one):
 //   2,304 outputs of 9,216    32 rows  32s 83*   48 rows  32s 114  48s 109*   64 rows  32s 114* (138)  48s 155  64s 138    90 rows  32s 152  48s 155*  64s 205
 //                            120 rows  32s 194* (208)  48s 203  64s 207  128s 258     200 rows  32s 301  48s 306*  64s 334 (334)  128s 386
-//                            700 rows  48s 798* (1,129)  64s 814  64 1,131  128 1,053  128s 1,037
+//                            700 rows  48s 798  64s 811* (1,129)  64 1,131  128 1,053  128s 1,037
 //   18,432 outputs of 2,304   48 rows  32s 171  48s 121*  64s 164   64 rows  32s 171  64s 165*  64 173   120 rows  32 317  64 294  128 277*    900 rows  48 1,984* (2,199)
 //   3,584 outputs of 14,336   64 rows  32s 235  64s 212*   128 rows  32s 415  64s 429 (429)  128s 396*   160 rows  32s 509* (603)  64s 604   512 rows  48s 1,385* (1,753)  128 1,627
 //   8,192 outputs of 3,584    96 rows  48s 165*   256 rows  32s 441  64s 419  128 421* (449)   384 rows  48s 588* (697)  64s 622  128 838
-//   256 outputs of 96         64 rows  32s 4.1* (5.9)  64s 5.9
-// Where it errs the sums are short, so that the meeting of a shared tile weighs more: 5,000 outputs of 300, 400 rows 80 us against 73.
-inline TileForm tile_form(int M, int N, int sms) {
+//   256 outputs of 96         64 rows  32s 4.1* (5.9)  64s 5.9          768 outputs of 3,072   600 rows  48s 102  128s 93*
+//   8,000 outputs of 300     400 rows  48s 123  64 108*      800 rows  48s 227  128 212*
+inline TileForm tile_form(int M, int N, int K, int sms) {
     TileForm best = {0, 0, false};
-    long long least = 0;
+    double least = 0;
     for (const TileCost& c : TILE_COSTS) {
         const long long down = ((long long)M + c.rows - 1) / c.rows, tiles = (N + (long long)BN - 1) / BN * down;
         if (down > 65535 && c.rows < 64) continue;               // the grid's height
         for (const bool shared : {true, false}) {
-            const long long cost = tile_cost(c, shared, tiles, sms);
+            const double cost = tile_cost(c, shared, tiles, K, sms);
             if (best.rows && cost >= least) continue;
             least = cost;
             // Three chunks, which leave room for two blocks a multiprocessor, where all tiles find room in that way and with two chunks
@@ -408,7 +412,7 @@ inline TileForm tile_form(int M, int N, int sms) {
 template <bool ALIGNED>
 cudaError_t launch_rows(float* out, const float* x, const float* w, int M, int N, int K, cudaStream_t st) {
     if (M <= FEW_MAX) return launch_few_rows<ALIGNED>(out, x, w, M, N, K, st);
-    const TileForm f = tile_form(M, N, rdl_sm_count());
+    const TileForm f = tile_form(M, N, K, rdl_sm_count());
     if (f.rows == 32) return !f.shared ? launch_tile<4, 8, 2, false, ALIGNED>(out, x, w, M, N, K, st)
                              : f.chunks == 2 ? launch_tile<4, 8, 2, true, ALIGNED>(out, x, w, M, N, K, st)
                                              : launch_tile<4, 8, 3, true, ALIGNED>(out, x, w, M, N, K, st);
@@ -423,9 +427,9 @@ cudaError_t launch_rows(float* out, const float* x, const float* w, int M, int N
 
 // The form a product takes on so many multiprocessors: 100 x rows of a tile + 10 x chunks of the ring + 1 where eight blocks share a tile;
 // 0: the few-row kernel.
-extern "C" int rdl_gemm_f32_form(int m, int n, int sms) {
+extern "C" int rdl_gemm_f32_form(int m, int n, int k, int sms) {
     if (m <= FEW_MAX) return 0;
-    const TileForm f = tile_form(m, n, sms);
+    const TileForm f = tile_form(m, n, k, sms);
     return 100 * f.rows + 10 * f.chunks + (f.shared ? 1 : 0);
 }
 

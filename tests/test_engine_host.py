@@ -262,18 +262,19 @@ def test_delta_rule_columns_follow_the_walk(tmp_path, monkeypatch):
 def test_tiles_of_the_32_bit_product_follow_the_waves():
     """Rows of a tile, chunks of the ring, and whether eight blocks share a tile, on 148 multiprocessors: short tiles where all find room
     at once, tall ones where fewer waves do; no ring that leaves room for fewer clusters than the tiles need."""
-    form = lambda m, n, sms=148: library.load().rdl_gemm_f32_form(m, n, sms)
+    form = lambda m, n, k=4096, sms=148: library.load().rdl_gemm_f32_form(m, n, k, sms)
     assert [form(m, 256) for m in (1, 16, 17, 64, 96)] == [0, 0, 3221, 3221, 3221]
     assert [form(m, 1000) for m in (96, 128)] == [3221, 3231]                      # 16 clusters of one block a multiprocessor do not find room
     assert [form(m, 2304) for m in (32, 48, 64, 96, 128, 200)] == [3221, 4821, 3221, 4821, 3221, 4821]
     assert [form(m, 4096) for m in (32, 48, 64, 128, 512)] == [3231, 4831, 6421, 6421, 12830]
     assert [form(m, 3584) for m in (112, 128, 512)] == [12831, 12831, 4821]
     assert [form(m, 18432) for m in (48, 64, 128)] == [4821, 6421, 12830]
+    assert [form(m, 8000, 300) for m in (400, 800)] == [6420, 12830]               # short sums: the meetings of shared tiles weigh more
     assert [form(48, 128 * n) // 10 % 10 for n in (24, 25, 33, 34)] == [2, 3, 3, 2]
     for m in (17, 32, 33, 64, 97, 300, 5000, 65535 * 48 + 1, 65535 * 64):
         for n in (1, 128, 129, 5000, 300000):
             for sms in (1, 8, 132, 148):
-                rows, rest = divmod(form(m, n, sms), 100)
+                rows, rest = divmod(form(m, n, 4096, sms), 100)
                 assert rows in (32, 48, 64, 128) and rest in (20, 21, 30, 31) and -(-m // rows) <= 65535, (m, n, sms)
 
 

@@ -147,7 +147,7 @@ def test_gemm_f32_sums_in_one_order_in_every_form(form):
     on this device, gives the few-row kernel's bits in its first and last columns; weights on and off 16-byte boundaries."""
     takes = library.load().rdl_gemm_f32_form
     sizes = [(m, n) for m in (17, 31, 33, 47, 50, 64, 97, 127, 160, 200, 299) for n in (1000, 3500, 6000, 12001, 16001, 18000, 25001, 36001, 50001, 75001)
-             if takes(m, n, ops.sm_count(0)) == form]
+             if takes(m, n, 300, ops.sm_count(0)) == form]
     assert sizes, form
     (m, n), k = min(sizes, key=lambda s: s[0] * s[1]), 300
     x, w = rnd((m, k), torch.float32, 3), rnd((n, k), torch.float32, n)
